@@ -44,13 +44,108 @@ int launch_box_field_fp64(int q, const Geo &g, const double *buf, int field, dou
 
 namespace {
 
-// Serial sum in index order: the reference's kinectic_energy loop (Other_functions.cpp:100-115).
-__global__ void k_sum_serial(const double *__restrict__ x, long long n, double *out)
+// Serial sum in index order: the reference's kinectic_energy loop (Other_functions.cpp:100-115), rounded
+// after every add as that loop is, by one warp.  One thread's chain of adds costs a load and an add
+// latency per element (4096 elements: 170 us).  While the sum s stays in one binade [2^e, 2^(e+1)), with unit
+// u = 2^(e-52), adding x >= 0 rounds to s + u rint(x / u): what each element adds is an integer multiple of u
+// that does not depend on s, except at a tie.  So a chunk of SER_CHUNK elements is rounded in parallel and summed
+// exactly in 64-bit integers by a warp scan, up to the first element that takes s out of its binade, ties, or
+// is not a non-negative finite number; that element is added by a plain FP64 add, and the chunk goes on
+// behind it.  A sum of n similar terms leaves its binade log2(n) times.  A chunk with more than SER_STOPS
+// such elements (ties on equal inputs) is finished by a plain loop.  erlbm_kinetic_energy, launches and
+// read-back included: 4096 nodes 218 -> 68 us, 16384 784 -> 120, 65536 3040 -> 329.
+constexpr int SER_PER_LANE = 8;
+constexpr int SER_CHUNK = 32 * SER_PER_LANE;
+constexpr int SER_STOPS = 24;
+
+__global__ void __launch_bounds__(32) k_sum_serial(const double *__restrict__ x, long long n, double *out)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    double s = 0;
-    for (long long i = 0; i < n; i++) s = s + x[i];
-    *out = s;
+    constexpr unsigned long long HIDDEN = 1ull << 52, MANT = HIDDEN - 1;
+    const int lane = threadIdx.x;
+    double s = 0.0;
+    double v[SER_PER_LANE], nx[SER_PER_LANE];
+    auto load = [&](long long base, double w[SER_PER_LANE]) {
+#pragma unroll
+        for (int j = 0; j < SER_PER_LANE; j++) {
+            const long long i = base + lane * SER_PER_LANE + j;
+            w[j] = i < n ? x[i] : 0.0;  // adding +0 changes nothing
+        }
+    };
+    load(0, nx);
+    for (long long base = 0; base < n; base += SER_CHUNK) {
+#pragma unroll
+        for (int j = 0; j < SER_PER_LANE; j++) v[j] = nx[j];
+        load(base + SER_CHUNK, nx);
+        int done = 0;  // elements of the chunk already in s
+        for (int stops = 0;; stops++) {
+            const unsigned long long sb = (unsigned long long)__double_as_longlong(s);
+            const int se = (int)(sb >> 52);  // 0 for s = 0, > 2046 for a negative, infinite or NaN sum
+            const bool in_binade = se >= 1 && se <= 2046;
+            if (stops == SER_STOPS || (se > 2046 && done == 0)) {
+                const int m = (int)(n - base < SER_CHUNK ? n - base : SER_CHUNK);
+                for (int i = done; i < m; i++) s = s + x[base + i];
+                break;
+            }
+            const unsigned long long S = in_binade ? (sb & MANT) | HIDDEN : 0ull;
+            // each element in units of u: q, and whether it has to be added on its own
+            unsigned long long q[SER_PER_LANE], sum = 0;
+            unsigned own = 0;
+#pragma unroll
+            for (int j = 0; j < SER_PER_LANE; j++) {
+                const bool todo = lane * SER_PER_LANE + j >= done;
+                const unsigned long long b = (unsigned long long)__double_as_longlong(v[j]);
+                const int xe = (int)(b >> 52);
+                const int sh = se - xe;
+                q[j] = 0;
+                if (todo && b != 0) {
+                    if (!in_binade || xe < 1 || sh < 0) {
+                        own |= 1u << j;  // no binade yet, subnormal, larger than s, negative or non-finite
+                    } else if (sh <= 53) {
+                        const unsigned long long m = (b & MANT) | HIDDEN;
+                        const unsigned long long half = sh ? 1ull << (sh - 1) : 0ull;
+                        const unsigned long long rem = sh ? m & ((1ull << sh) - 1) : 0ull;
+                        q[j] = (m >> sh) + (rem > half ? 1ull : 0ull);
+                        if (sh && rem == half) own |= 1u << j;
+                    }
+                }
+                sum += q[j];
+            }
+            unsigned long long incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            // the lane's first element that cannot be taken, with the sum before it
+            unsigned long long acc = S + (incl - sum), at = 0;
+            int stop = SER_PER_LANE;
+#pragma unroll
+            for (int j = 0; j < SER_PER_LANE; j++) {
+                if (stop == SER_PER_LANE && (((own >> j) & 1u) || acc + q[j] >= 2 * HIDDEN)) {
+                    stop = j;
+                    at = acc;
+                }
+                acc += q[j];
+            }
+            const unsigned who = __ballot_sync(0xffffffffu, stop < SER_PER_LANE);
+            if (who == 0) {
+                const unsigned long long total = __shfl_sync(0xffffffffu, acc, 31);
+                if (in_binade) s = __longlong_as_double((long long)((total & MANT) | ((unsigned long long)se << 52)));
+                break;
+            }
+            const int first = __ffs(who) - 1;
+            const unsigned long long before = __shfl_sync(0xffffffffu, at, first);
+            double mine = 0.0;
+#pragma unroll
+            for (int j = 0; j < SER_PER_LANE; j++)
+                if (j == stop) mine = v[j];
+            const double xs = __shfl_sync(0xffffffffu, mine, first);
+            if (in_binade) s = __longlong_as_double((long long)((before & MANT) | ((unsigned long long)se << 52)));
+            s = s + xs;
+            done = first * SER_PER_LANE + __shfl_sync(0xffffffffu, stop, first) + 1;
+        }
+    }
+    if (lane == 0) *out = s;
 }
 
 constexpr int RB = 256;   // threads per reduction block
@@ -113,16 +208,28 @@ __global__ void __launch_bounds__(RB) k_maxabs_partial(const double *__restrict_
     }
 }
 
-__global__ void k_maxabs_final(const double *__restrict__ part, double *out)
+__global__ void __launch_bounds__(RB) k_maxabs_final(const double *__restrict__ part, double *out)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    __shared__ double sm[RB], sf[RB];
     double m = 0, nf = 0;
-    for (int i = 0; i < RG; i++) {
+    for (int i = threadIdx.x; i < RG; i += RB) {
         m = fmax(m, part[2 * i]);
         nf = fmax(nf, part[2 * i + 1]);
     }
-    out[0] = m;
-    out[1] = nf;
+    sm[threadIdx.x] = m;
+    sf[threadIdx.x] = nf;
+    __syncthreads();
+    for (int o = RB / 2; o > 0; o >>= 1) {
+        if (threadIdx.x < o) {
+            sm[threadIdx.x] = fmax(sm[threadIdx.x], sm[threadIdx.x + o]);
+            sf[threadIdx.x] = fmax(sf[threadIdx.x], sf[threadIdx.x + o]);
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        out[0] = sm[0];
+        out[1] = sf[0];
+    }
 }
 
 }  // namespace
@@ -141,7 +248,7 @@ int launch_sum(const double *x, long long n, long long serial_limit, double *scr
 int launch_maxabs(const double *x, long long n, double *scratch, double *out, cudaStream_t s)
 {
     k_maxabs_partial<<<RG, RB, 0, s>>>(x, n, scratch);
-    k_maxabs_final<<<1, 32, 0, s>>>(scratch, out);
+    k_maxabs_final<<<1, RB, 0, s>>>(scratch, out);
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
