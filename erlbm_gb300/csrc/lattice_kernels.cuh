@@ -552,6 +552,14 @@ __global__ void __launch_bounds__(256) k_box_field(Geo g, const typename P::T *_
 
 inline unsigned blocks_for(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
+// Threads per block of the per-node kernels.  FP64: 64, at every size.  They are bound by the FP64 pipe, a
+// quarter of which belongs to each scheduler of an SM: a small lattice has to reach as many schedulers as it
+// has warps (3936 nodes: 16 blocks of 256 leave 136 SMs idle, 62 blocks of 64 use two schedulers on 62), and a
+// large one ends with a shorter last wave.  82 x 48 D3Q19: 32.0 -> 15.5 us a step, 64^2 D2Q9 16.5 -> 8.3;
+// 512^2 and 64^3: 1-2 % of the step.
+template <class P>
+constexpr int node_block = sizeof(typename P::T) == 8 ? 64 : 256;
+
 template <class P>
 int box_field_any(int q, const Geo &g, const typename P::T *buf, int field, double *out, cudaStream_t s)
 {
@@ -572,23 +580,24 @@ int step_dispatch(int op, const Geo &g, const BCp &bc, const Relax &R, const Ste
     CollParams prm;
     prm.R = R;
     prm.k = shifted::make_coef(R);
-    const unsigned nb = blocks_for(g.nbox, 256);
+    constexpr int bs = node_block<P>;
+    const unsigned nb = blocks_for(g.nbox, bs);
     switch (op) {
     case OP_BGK:
-        k_step<P, Q, OP_BGK><<<nb, 256, 0, s>>>(src, dst, g, bc, prm, a);
+        k_step<P, Q, OP_BGK><<<nb, bs, 0, s>>>(src, dst, g, bc, prm, a);
         break;
     case OP_MRT:
         if constexpr (Q == 9) {
-            k_step<P, Q, OP_MRT><<<nb, 256, 0, s>>>(src, dst, g, bc, prm, a);
+            k_step<P, Q, OP_MRT><<<nb, bs, 0, s>>>(src, dst, g, bc, prm, a);
             break;
         } else {
             return -1;
         }
     case OP_REG:
-        k_step<P, Q, OP_REG><<<nb, 256, 0, s>>>(src, dst, g, bc, prm, a);
+        k_step<P, Q, OP_REG><<<nb, bs, 0, s>>>(src, dst, g, bc, prm, a);
         break;
     case OP_EXTREG:
-        k_step<P, Q, OP_EXTREG><<<nb, 256, 0, s>>>(src, dst, g, bc, prm, a);
+        k_step<P, Q, OP_EXTREG><<<nb, bs, 0, s>>>(src, dst, g, bc, prm, a);
         break;
     default:
         return -1;
@@ -653,11 +662,12 @@ int node_fields_any(int q, const Geo &g, long long n, const int *nof, const type
                     double *rho, double *u, cudaStream_t s)
 {
     if (n == 0) return 0;
-    const unsigned nb = blocks_for(n, 256);
+    constexpr int bs = node_block<P>;
+    const unsigned nb = blocks_for(n, bs);
     if (q == 9)
-        k_node_fields<P, 9><<<nb, 256, 0, s>>>(g, n, nof, buf, e, rho, u);
+        k_node_fields<P, 9><<<nb, bs, 0, s>>>(g, n, nof, buf, e, rho, u);
     else if (q == 19)
-        k_node_fields<P, 19><<<nb, 256, 0, s>>>(g, n, nof, buf, e, rho, u);
+        k_node_fields<P, 19><<<nb, bs, 0, s>>>(g, n, nof, buf, e, rho, u);
     else
         return -1;
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
