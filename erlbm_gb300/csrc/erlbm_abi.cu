@@ -83,6 +83,7 @@ struct erlbm_handle {
     RunStatus *d_status = nullptr;
     cudaStream_t stream = nullptr;
     cudaStream_t own_stream = nullptr;  // the stream created at erlbm_create
+    bool own_shape = true;              // no erlbm_set_launch call: the engine chooses the launch shape
     int shape = 0;                      // launch shape of the fused periodic kernel (erlbm_set_launch)
     bool two_step = false;              // pairs of fused periodic steps as one launch (erlbm_set_launch)
     bool three_step = false;            // triples of fused periodic steps as one launch (erlbm_set_launch)
@@ -369,6 +370,45 @@ int enqueue_step(erlbm_handle *h, const BCp &bc, int check_density, double densi
     return ERLBM_OK;
 }
 
+// How plain periodic FP32-shifted D2Q9 steps are launched: steps per launch (1 where the multi-step strips do
+// not apply), 64-column strips for three steps, and whether single steps have the fused kernel.
+struct PeriodicPlan {
+    int per_launch = 1;
+    bool wide = false, fused1 = false;
+};
+
+// erlbm_set_launch's shape on the boxes it takes (nx % 128 == 0, and ny even for several steps); otherwise
+// three steps per launch wherever the strips fit.  They are the fastest form from the smallest box on, us per
+// step against one step per launch (the fused kernel; the generic one where nx % 128 != 0): 128^2 2.1 / 2.6,
+// 512^2 2.8 / 3.8, 1024^2 6.8 / 8.5, 2048^2 19.3 / 45.3; 100^2 2.1 / 4.1, 1001 x 618 4.8 / 12.3, 2047^2
+// 23.6 / 75.8.  Two steps per launch lie between (2.3, 3.1, 7.7, 29.4).
+PeriodicPlan periodic_plan(const erlbm_handle *h)
+{
+    PeriodicPlan p;
+    p.fused1 = periodic_d2q9_fp32_ok(h->g);
+    if (!h->own_shape && p.fused1) {
+        if (h->three_step && periodic_d2q9_x2_ok(h->g) && (!h->wide_strips || periodic_d2q9_x3a_ok(h->g))) {
+            p.per_launch = 3;
+            p.wide = h->wide_strips;
+        } else if (h->two_step && periodic_d2q9_x2_ok(h->g)) {
+            p.per_launch = 2;
+        }
+    } else if (periodic_d2q9_strips_ok(h->g)) {
+        p.per_launch = 3;
+        p.wide = periodic_d2q9_prefers_wide(h->g);
+    }
+    return p;
+}
+
+// per_launch (1, 2 or 3) plain periodic steps as one launch.
+int launch_periodic(const erlbm_handle *h, const PeriodicPlan &p, int steps, const float *src, float *dst,
+                    cudaStream_t s)
+{
+    if (steps == 3) return launch_periodic_d2q9_fp32_x3(h->op, h->g, h->R, src, dst, s, p.wide);
+    if (steps == 2) return launch_periodic_d2q9_fp32_x2(h->op, h->g, h->R, src, dst, s);
+    return launch_periodic_d2q9_fp32(h->op, h->g, h->R, src, dst, s, h->shape);
+}
+
 // A block of plain periodic steps of the fused FP32 D2Q9 kernels (per_launch steps per launch) as one
 // CUDA graph launch: the launches of a block are captured once per buffer parity and replayed, so a
 // small lattice is not bound by the host's launch rate.  An even number of launches leaves the
@@ -376,10 +416,10 @@ int enqueue_step(erlbm_handle *h, const BCp &bc, int check_density, double densi
 // steps per graph: an even number of launches of every shape (1, 2 or 3 steps each)
 int graph_steps_of(int per_launch) { return per_launch == 3 ? 66 : 64; }
 
-int graph_steps(erlbm_handle *h, int per_launch)
+int graph_steps(erlbm_handle *h, const PeriodicPlan &p)
 {
-    const int n_steps = graph_steps_of(per_launch);
-    const long long key = per_launch | ((long long)h->shape << 2);
+    const int n_steps = graph_steps_of(p.per_launch);
+    const long long key = p.per_launch | (p.wide ? 4 : 0) | ((long long)h->shape << 3);
     if (h->graph_key != key) {
         drop_graphs(h);
         h->graph_key = key;
@@ -389,14 +429,9 @@ int graph_steps(erlbm_handle *h, int per_launch)
         if (!h->capture_stream) CK(cudaStreamCreateWithFlags(&h->capture_stream, cudaStreamNonBlocking));
         CK(cudaStreamBeginCapture(h->capture_stream, cudaStreamCaptureModeRelaxed));
         int c = h->cur, lrc = 0;
-        for (int k = 0; k < n_steps / per_launch && lrc == 0; k++) {
-            const float *src = (const float *)h->d_buf[c];
-            float *dst = (float *)h->d_buf[c ^ 1];
-            lrc = per_launch == 3   ? launch_periodic_d2q9_fp32_x3(h->op, h->g, h->R, src, dst, h->capture_stream,
-                                                                 h->wide_strips)
-                  : per_launch == 2 ? launch_periodic_d2q9_fp32_x2(h->op, h->g, h->R, src, dst, h->capture_stream)
-                                    : launch_periodic_d2q9_fp32(h->op, h->g, h->R, src, dst, h->capture_stream,
-                                                                h->shape);
+        for (int k = 0; k < n_steps / p.per_launch && lrc == 0; k++) {
+            lrc = launch_periodic(h, p, p.per_launch, (const float *)h->d_buf[c], (float *)h->d_buf[c ^ 1],
+                                  h->capture_stream);
             c ^= 1;
         }
         cudaGraph_t graph = nullptr;
@@ -466,6 +501,46 @@ int bc_graph_steps(erlbm_handle *h, const BCp &b)
     CK(cudaGraphLaunch(x, h->stream));
     h->steps_done += BC_GRAPH_STEPS;
     h->kind = 1;
+    return ERLBM_OK;
+}
+
+// n_steps steps without checks, by graph blocks and multi-step launches where they apply.
+int advance(erlbm_handle *h, int n_steps, const BCp &b)
+{
+    int rc;
+    const bool fp32_2d = h->prec == ERLBM_FP32_SHIFTED && h->q == 9;
+    const bool plain = fp32_2d && b.inlet_x < 0 && b.outlet_x < 0 && b.open_y < 0 && h->g.solid == nullptr;
+    PeriodicPlan p;
+    if (plain) p = periodic_plan(h);
+    const bool hybrid = fp32_2d && !plain && d2q9_hybrid_ok(h->g);
+    for (int s = 0; s < n_steps;) {
+        const int left = n_steps - s;
+        if (hybrid && h->kind == 1 && left >= BC_GRAPH_STEPS) {
+            if ((rc = bc_graph_steps(h, b))) return rc;
+            s += BC_GRAPH_STEPS;
+            continue;
+        }
+        if (plain && h->kind == 1 && (p.per_launch > 1 || p.fused1)) {
+            if (left >= graph_steps_of(p.per_launch)) {
+                if ((rc = graph_steps(h, p))) return rc;
+                s += graph_steps_of(p.per_launch);
+                continue;
+            }
+            // a launch of the plan's steps, or of the two that a three-step plan chosen here has left
+            const int m = left >= p.per_launch ? p.per_launch
+                          : (left == 2 && h->own_shape && periodic_d2q9_strips_ok(h->g)) ? 2 : 1;
+            if (m > 1) {
+                CKL(launch_periodic(h, p, m, (const float *)h->d_buf[h->cur], (float *)h->d_buf[h->cur ^ 1], h->stream),
+                    "periodic_d2q9");
+                h->cur ^= 1;
+                h->steps_done += m;
+                s += m;
+                continue;
+            }
+        }
+        if ((rc = enqueue_step(h, b, 0, 0.0, false))) return rc;
+        s++;
+    }
     return ERLBM_OK;
 }
 
@@ -720,48 +795,7 @@ int erlbm_step(erlbm_handle *h, int n_steps, const erlbm_bc *bc)
     if (n_steps < 0) return ERLBM_E_INVAL;
     BCp b;
     if ((rc = validate_bc(h, bc, &b))) return rc;
-    const bool plain = h->prec == ERLBM_FP32_SHIFTED && h->q == 9 && b.inlet_x < 0 && b.outlet_x < 0 &&
-                       b.open_y < 0 && periodic_d2q9_fp32_ok(h->g);
-    const bool fused3 = plain && h->three_step && periodic_d2q9_x2_ok(h->g) &&
-                        (!h->wide_strips || periodic_d2q9_x3a_ok(h->g));
-    const bool fused2 = plain && h->two_step && periodic_d2q9_x2_ok(h->g);
-    const int per_launch = fused3 ? 3 : (fused2 ? 2 : 1);
-    const bool hybrid = !plain && h->prec == ERLBM_FP32_SHIFTED && h->q == 9 && d2q9_hybrid_ok(h->g);
-    for (int s = 0; s < n_steps;) {
-        if (hybrid && h->kind == 1 && n_steps - s >= BC_GRAPH_STEPS) {
-            if ((rc = bc_graph_steps(h, b))) return rc;
-            s += BC_GRAPH_STEPS;
-            continue;
-        }
-        if (plain && h->kind == 1 && n_steps - s >= graph_steps_of(per_launch)) {
-            if ((rc = graph_steps(h, per_launch))) return rc;
-            s += graph_steps_of(per_launch);
-            continue;
-        }
-        if (fused3 && h->kind == 1 && n_steps - s >= 3) {
-            // three plain periodic steps in one launch
-            CKL(launch_periodic_d2q9_fp32_x3(h->op, h->g, h->R, (const float *)h->d_buf[h->cur],
-                                             (float *)h->d_buf[h->cur ^ 1], h->stream, h->wide_strips),
-                "periodic_d2q9_x3");
-            h->cur ^= 1;
-            h->steps_done += 3;
-            s += 3;
-            continue;
-        }
-        if (fused2 && h->kind == 1 && n_steps - s >= 2) {
-            // two plain periodic steps in one launch: step s and s + 1
-            CKL(launch_periodic_d2q9_fp32_x2(h->op, h->g, h->R, (const float *)h->d_buf[h->cur],
-                                             (float *)h->d_buf[h->cur ^ 1], h->stream),
-                "periodic_d2q9_x2");
-            h->cur ^= 1;
-            h->steps_done += 2;
-            s += 2;
-            continue;
-        }
-        if ((rc = enqueue_step(h, b, 0, 0.0, false))) return rc;
-        s++;
-    }
-    return ERLBM_OK;
+    return advance(h, n_steps, b);
 }
 
 int erlbm_set_launch(erlbm_handle *h, int block_threads, int flags)
@@ -783,6 +817,7 @@ int erlbm_set_launch(erlbm_handle *h, int block_threads, int flags)
         set_error("set_launch: at most one of ERLBM_LAUNCH_TWO_STEP and ERLBM_LAUNCH_THREE_STEP%s%s", "", "");
         return ERLBM_E_INVAL;
     }
+    h->own_shape = false;
     h->shape = block_threads | ((flags & ERLBM_LAUNCH_STREAMING_STORES) ? 0x1000 : 0) |
                ((flags & ERLBM_LAUNCH_WIDE_STRIPS) ? 0x2000 : 0);  // part of the graph key
     h->two_step = (flags & ERLBM_LAUNCH_TWO_STEP) != 0;
@@ -896,6 +931,11 @@ int erlbm_run(erlbm_handle *h, int n_steps, const erlbm_bc *bc, const erlbm_chec
         }
         int m = chunk - (s % chunk);
         if (s + m > n_steps) m = n_steps - s;
+        if (!c.density_check) {
+            if ((rc = advance(h, m, b))) return rc;
+            s += m;
+            continue;
+        }
         // keep the step numbering of the run itself in the kernels' step index
         for (int k = 0; k < m; k++) {
             h->steps_done = base + s + k;

@@ -19,6 +19,7 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
+
 // Pull one direction plane for the four nodes x0..x0+3 of row y (periodic in x and y).
 template <int CX>
 __device__ __forceinline__ float4 pull4(const float *__restrict__ row, int x0, int xl, int xr, int lane)
@@ -276,10 +277,11 @@ __global__ void __launch_bounds__(128) k_periodic_d2q9_x2s(const float *__restri
         shifted::collide9x2<OP>(g, k);
         if (store) {
             float *d0 = dst + (long long)j * nx + c, *d1 = d0 + nx;
+            const bool second = j + 1 < y1;  // an odd chunk's last iteration stores one row
 #pragma unroll
             for (int i = 0; i < 9; i++) {
                 d0[i * plane] = g[i].x;
-                d1[i * plane] = g[i].y;
+                if (second) d1[i * plane] = g[i].y;
             }
         }
 #pragma unroll
@@ -446,10 +448,11 @@ __global__ void __launch_bounds__(128, 4) k_periodic_d2q9_x3s(const float *__res
         shifted::collide9x2<OP>(g, k);
         if (store) {
             float *d0 = dst + (long long)j * nx + c, *d1 = d0 + nx;
+            const bool second = j + 1 < y1;  // an odd chunk's last iteration stores one row
 #pragma unroll
             for (int i = 0; i < 9; i++) {
                 d0[i * plane] = g[i].x;
-                d1[i * plane] = g[i].y;
+                if (second) d1[i * plane] = g[i].y;
             }
         }
 #pragma unroll
@@ -648,6 +651,12 @@ bool periodic_d2q9_x2_ok(const Geo &g)
     return periodic_d2q9_fp32_ok(g) && g.ny >= 4 && g.ny % 2 == 0;  // nx % 128 == 0 from the one-step check
 }
 
+// The scalar warp strips on any periodic box: a strip's columns and a chunk's rows wrap at most once.
+bool periodic_d2q9_strips_ok(const Geo &g)
+{
+    return g.solid == nullptr && g.nz == 1 && g.nx >= 32 && g.ny >= 8;
+}
+
 // Two-step launch: 128-thread CTAs of four independent warps, and rows per chunk such that one wave
 // of resident warps covers the ceil(nx / 30) x (ny / hc) warp strips (no second, partial wave).
 template <int OP>
@@ -747,16 +756,46 @@ static void go_x3a(const Geo &g, const shifted::Coef &k, const float *src, float
 
 bool periodic_d2q9_x3a_ok(const Geo &g)
 {
-    // 64-column strips need ny >= 16; the nine planes are addressed with 32-bit offsets
-    return periodic_d2q9_fp32_ok(g) && g.ny >= 16 && g.nx >= 128 && 9 * g.plane < (1LL << 31);
+    // 64-column strips need ny >= 16; 16-byte copies start at multiples of four columns of any row; the nine
+    // planes are addressed with 32-bit offsets
+    return g.solid == nullptr && g.nz == 1 && g.nx % 4 == 0 && g.ny >= 16 && g.nx >= 128 && 9 * g.plane < (1LL << 31);
 }
 
-// Three steps of the fused periodic D2Q9 FP32 update in one launch (periodic_d2q9_x2_ok(g) required;
+// Rows per chunk of a three-step launch: one wave of `resident` warps covers the strips.
+static long long x3_rows(const Geo &g, long long resident, int width, int multiple, int least)
+{
+    const long long strips = (g.nx + width - 1) / width;
+    const long long chunks = resident / strips > 0 ? resident / strips : 1;
+    long long hc = (g.ny + chunks - 1) / chunks;
+    hc = (hc + multiple - 1) / multiple * multiple;
+    return hc < least ? least : hc;
+}
+
+// The two three-step kernels keep the same 16 warps per SM, and a warp iteration of either collides one float2
+// per lane and stage, so a launch takes (iterations of a warp) x (time of an iteration): rows + 2 of prologue
+// at 1.85 us (64-column strips: 2048^2 57.8 us / 32, 1024^2 21.2 / 11), row pairs + 1 at 2.2 us (32-column:
+// 70.7 / 33, 20.2 / 9).  Measured, us per step, 64- against 32-column strips: 512^2 3.32 / 2.77, 512 x 1024
+// 4.33 / 4.13, 1024^2 7.05 / 6.75, 1536 x 1024 8.78 / 9.72, 1536^2 12.2 / 14.2, 2048^2 19.3 / 23.6, 4096^2
+// 76.5 / 87.2; the estimate picks the faster one in all of these (768^2, 4.35 / 4.79, it misses).
+bool periodic_d2q9_prefers_wide(const Geo &g)
+{
+    if (!periodic_d2q9_x3a_ok(g)) return false;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return false;
+    const long long resident = 16LL * sms;
+    const double wide = (double)(x3_rows(g, resident, XP_W, XP_SPAN, 2 * XP_SPAN) + 2) * 1.85;
+    const double narrow = (double)(x3_rows(g, resident, X3_W, 2, 8) / 2 + 1) * 2.2;
+    return wide < narrow;
+}
+
+// Three steps of the fused periodic D2Q9 FP32 update in one launch (periodic_d2q9_strips_ok(g) or _x2_ok(g) required;
 // wide = the column-pair kernel, which needs periodic_d2q9_x3a_ok(g)).
 int launch_periodic_d2q9_fp32_x3(int op, const Geo &g, const Relax &R, const float *src, float *dst, cudaStream_t s,
                                  bool wide)
 {
-    if (!periodic_d2q9_x2_ok(g) || (wide && !periodic_d2q9_x3a_ok(g))) return -1;
+    if (!(wide ? periodic_d2q9_x3a_ok(g) : periodic_d2q9_strips_ok(g) || periodic_d2q9_x2_ok(g))) return -1;
     const shifted::Coef k = shifted::make_coef(R);
     if (wide) {
         switch (op) {
@@ -778,10 +817,10 @@ int launch_periodic_d2q9_fp32_x3(int op, const Geo &g, const Relax &R, const flo
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-// Two steps of the fused periodic D2Q9 FP32 update in one launch (periodic_d2q9_x2_ok(g) required).
+// Two steps of the fused periodic D2Q9 FP32 update in one launch (periodic_d2q9_strips_ok(g) or _x2_ok(g) required).
 int launch_periodic_d2q9_fp32_x2(int op, const Geo &g, const Relax &R, const float *src, float *dst, cudaStream_t s)
 {
-    if (!periodic_d2q9_x2_ok(g)) return -1;
+    if (!periodic_d2q9_strips_ok(g) && !periodic_d2q9_x2_ok(g)) return -1;
     const shifted::Coef k = shifted::make_coef(R);
     switch (op) {
     case OP_BGK: go_x2<OP_BGK>(g, k, src, dst, s); break;

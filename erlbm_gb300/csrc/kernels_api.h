@@ -66,6 +66,10 @@ bool periodic_d2q9_x2_ok(const Geo &g);
 int launch_periodic_d2q9_fp32_x3(int op, const Geo &g, const Relax &R, const float *src, float *dst, cudaStream_t s,
                                  bool wide);
 bool periodic_d2q9_x3a_ok(const Geo &g);
+// The two-step and the 32-column three-step strips on any periodic box (nx >= 32, ny >= 8, any remainder).
+bool periodic_d2q9_strips_ok(const Geo &g);
+// Launch of three steps that runs the box faster: true = the 64-column strips.
+bool periodic_d2q9_prefers_wide(const Geo &g);
 
 // Stream only: dst = post-stream populations of the post-collision state src (no BC, no collision).
 int launch_stream_only_fp64(int q, const Geo &g, const double *src, double *dst, cudaStream_t s);

@@ -40,3 +40,38 @@ def test_energy_sum_keeps_the_serial_order_and_rounding(nx, ny, kind):
         lat.set_populations(f)
         a, b = lat.kinetic_energy(E.STAGE_POST_STREAM), ref.kinetic_energy(0)
         assert a == b or (np.isnan(a) and np.isnan(b))
+
+
+@pytest.mark.parametrize("nx,ny", [(32, 8), (33, 9), (61, 17), (128, 19), (132, 16), (190, 31), (1001, 24), (644, 70),
+                                   (1996, 401)])
+@pytest.mark.parametrize("steps", [2, 3, 6, 73])
+def test_periodic_steps_of_any_box_equal_their_cpu_restatement(nx, ny, steps):
+    """Two- and three-step strips chosen by the engine, on boxes whose sides leave remainders of the strips,
+    chunks and row pairs; leftover steps; graph blocks (73 steps)."""
+    import erlbm_gb300 as E
+    if nx * ny * steps > 6e6:
+        steps = 7
+    op = (1, 3, 4, 2)[(nx + ny + steps) % 4]
+    f = flow(9, nx, min(ny, 40), 1, nx)
+    f = np.resize(f.reshape(-1, 9), (nx * ny, 9)).reshape(-1)
+    tnh = 1.0 if op == 3 else 0.65
+    with E.Lattice(9, nx, ny, 1, None, 0.53, tnh, op, E.FP32_SHIFTED) as lat:
+        lat.set_populations(f)
+        lat.step(steps)
+        got = lat.get_populations(E.STAGE_POST_COLLISION)
+    assert np.array_equal(got, O.fp32_periodic_d2q9(nx, ny, op, 0.53, tnh, f, steps))
+
+
+def test_run_without_density_checks_takes_the_stepping_path():
+    """run() with energy checks steps as step() does: the same populations, and the checks of the oracle's loop."""
+    import erlbm_gb300 as E
+    nx, ny = 132, 20
+    f = flow(9, nx, ny, 1, 3)
+    with E.Lattice(9, nx, ny, 1, None, 0.56, 0.65, 4, E.FP32_SHIFTED) as a, \
+            E.Lattice(9, nx, ny, 1, None, 0.56, 0.65, 4, E.FP32_SHIFTED) as b:
+        a.set_populations(f)
+        b.set_populations(f)
+        r = a.run(250, energy_every=100, energy_factor=50.0)
+        b.step(250)
+        assert r["label"] == 0 and r["steps_done"] == 250
+        assert np.array_equal(a.get_populations(), b.get_populations())
