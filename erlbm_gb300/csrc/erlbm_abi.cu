@@ -359,6 +359,9 @@ int enqueue_step(erlbm_handle *h, const BCp &bc, int check_density, double densi
         CKL(launch_step_fp32_hybrid(h->op, h->g, bc, h->R, (const float *)src, (float *)dst, h->d_segflag,
                                     h->d_nodeflag, h->d_fix, h->n_fix, h->stream),
             "d2q9_hybrid");
+    } else if (h->prec == ERLBM_FP32_SHIFTED && h->q == 19 && plain && periodic_d3q19_fp32_ok(h->g)) {
+        CKL(launch_periodic_d3q19_fp32(h->op, h->g, h->R, (const float *)src, (float *)dst, h->stream),
+            "periodic_d3q19");
     } else if (h->prec == ERLBM_FP64) {
         CKL(launch_step_fp64(h->q, h->op, h->g, bc, h->R, a, (const double *)src, (double *)dst, h->stream), "step");
     } else {

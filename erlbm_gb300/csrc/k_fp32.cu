@@ -861,6 +861,77 @@ int launch_periodic_d2q9_fp32(int op, const Geo &g, const Relax &R, const float 
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
+namespace {
+
+// Division of n < 2^31 by a launch constant d: (n m) >> (31 + sh) with m = ceil(2^(31 + sh) / d), 2^sh >= d.
+struct FastDiv {
+    unsigned d, m, sh;
+};
+FastDiv make_fastdiv(unsigned d)
+{
+    unsigned sh = 0;
+    while ((1ull << sh) < d) sh++;
+    return FastDiv{d, (unsigned)(((1ull << (31 + sh)) + d - 1) / d), sh};
+}
+__device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv &f)
+{
+    return (unsigned)(((unsigned long long)n * f.m) >> (31 + f.sh));
+}
+
+// One step of a periodic D3Q19 lattice without solids or planes, a node per thread.  Bound by HBM: every
+// population is read and written once (152 bytes per update; a population is pulled by one node only, so
+// there is nothing for a tile to share).  The generic kernel tests for a solid mask between its reads and
+// adds 64-bit offsets per direction; here all 19 reads are issued together, offsets are 32-bit and plane
+// bases uniform, and 128-thread blocks at 6 per SM keep 24 warps of reads in flight.  128^3: 71.3 -> 50.2 us
+// (4470 -> 6350 GB/s), 192^3: 226.8 -> 158.2 us (6800 GB/s, the measured copy rate), 64^3 (in L2): 10.3 ->
+// 8.3 us; 32^3 and below stay at the launch rate.
+template <int OP>
+__global__ void __launch_bounds__(128, 6) k_periodic_d3q19(const float *__restrict__ src, float *__restrict__ dst,
+                                                            unsigned nx, unsigned ny, unsigned nz, unsigned nbox,
+                                                            size_t plane, FastDiv fx, FastDiv fy, shifted::Coef k)
+{
+    const unsigned node = blockIdx.x * 128u + threadIdx.x;
+    if (node >= nbox) return;
+    const unsigned r = fdiv(node, fx), x = node - r * nx, z = fdiv(r, fy), y = r - z * ny;
+    const unsigned nxy = nx * ny;
+    // offsets (modulo 2^32) to the pulled node: from x - 1 for c_x = +1, and so on
+    const unsigned xm = x == 0 ? nx - 1 : 0u - 1u, xp = x == nx - 1 ? 1u - nx : 1u;
+    const unsigned ym = y == 0 ? nxy - nx : 0u - nx, yp = y == ny - 1 ? nx - nxy : nx;
+    const unsigned zm = z == 0 ? nxy * (nz - 1) : 0u - nxy, zp = z == nz - 1 ? 0u - nxy * (nz - 1) : nxy;
+    float f[19];
+#pragma unroll
+    for (int i = 0; i < 19; i++) {
+        const int cx = Lat<19>::cx(i), cy = Lat<19>::cy(i), cz = Lat<19>::cz(i);
+        const unsigned s = node + (cx == 1 ? xm : (cx == -1 ? xp : 0u)) + (cy == 1 ? ym : (cy == -1 ? yp : 0u)) +
+                           (cz == 1 ? zm : (cz == -1 ? zp : 0u));
+        f[i] = __ldg(src + (size_t)i * plane + s);
+    }
+    shifted::collide<19, OP>(f, k);
+#pragma unroll
+    for (int i = 0; i < 19; i++) dst[(size_t)i * plane + node] = f[i];
+}
+
+}  // namespace
+
+bool periodic_d3q19_fp32_ok(const Geo &g) { return g.solid == nullptr && g.nbox < (1LL << 30); }
+
+int launch_periodic_d3q19_fp32(int op, const Geo &g, const Relax &R, const float *src, float *dst, cudaStream_t s)
+{
+    if (!periodic_d3q19_fp32_ok(g)) return -1;
+    const shifted::Coef k = shifted::make_coef(R);
+    const unsigned nb = blocks_for(g.nbox, 128), n = (unsigned)g.nbox;
+    const FastDiv fx = make_fastdiv((unsigned)g.nx), fy = make_fastdiv((unsigned)g.ny);
+    const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny, nz = (unsigned)g.nz;
+    const size_t pl = (size_t)g.plane;
+    switch (op) {
+    case OP_BGK: k_periodic_d3q19<OP_BGK><<<nb, 128, 0, s>>>(src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
+    case OP_REG: k_periodic_d3q19<OP_REG><<<nb, 128, 0, s>>>(src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
+    case OP_EXTREG: k_periodic_d3q19<OP_EXTREG><<<nb, 128, 0, s>>>(src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
+    default: return -1;
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
 int launch_step_fp32(int q, int op, const Geo &g, const BCp &bc, const Relax &R, const StepArgs &a, const float *src,
                      float *dst, cudaStream_t s)
 {

@@ -71,6 +71,10 @@ bool periodic_d2q9_strips_ok(const Geo &g);
 // Launch of three steps that runs the box faster: true = the 64-column strips.
 bool periodic_d2q9_prefers_wide(const Geo &g);
 
+// One step of a periodic D3Q19 box in FP32-shifted (the generic kernel's bits).
+bool periodic_d3q19_fp32_ok(const Geo &g);
+int launch_periodic_d3q19_fp32(int op, const Geo &g, const Relax &R, const float *src, float *dst, cudaStream_t s);
+
 // Stream only: dst = post-stream populations of the post-collision state src (no BC, no collision).
 int launch_stream_only_fp64(int q, const Geo &g, const double *src, double *dst, cudaStream_t s);
 int launch_stream_only_fp32(int q, const Geo &g, const float *src, float *dst, cudaStream_t s);

@@ -62,6 +62,19 @@ def test_periodic_steps_of_any_box_equal_their_cpu_restatement(nx, ny, steps):
     assert np.array_equal(got, O.fp32_periodic_d2q9(nx, ny, op, 0.53, tnh, f, steps))
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1), (2, 1, 3), (129, 3, 2), (31, 33, 5), (127, 2, 7), (16, 16, 1)])
+@pytest.mark.parametrize("op", [1, 3, 4])
+def test_periodic_d3q19_of_any_box_equals_its_cpu_restatement(shape, op):
+    import erlbm_gb300 as E
+    f = flow(19, *shape, seed=sum(shape))
+    tnh = 1.0 if op == 3 else 0.65
+    with E.Lattice(19, *shape, None, 0.53, tnh, op, E.FP32_SHIFTED) as lat:
+        lat.set_populations(f)
+        lat.step(5)
+        got = lat.get_populations(E.STAGE_POST_COLLISION)
+    assert np.array_equal(got, O.fp32_periodic_d3q19(*shape, op, 0.53, tnh, f, 5))
+
+
 def test_run_without_density_checks_takes_the_stepping_path():
     """run() with energy checks steps as step() does: the same populations, and the checks of the oracle's loop."""
     import erlbm_gb300 as E
