@@ -487,9 +487,10 @@ __device__ __forceinline__ void zou_he_d2q9(float g[9], double vx)
     const double vx3 = __dmul_rn(3.0, vx);
     const double P = __dadd_rn(__dadd_rn(1.0, vx3), __dmul_rn(vx3, vx));
     const double e = __dadd_rn(__dmul_rn(rho, P), -1.0);
-    g[1] = (float)(e / 9.0);
-    g[5] = (float)(e / 36.0);
-    g[7] = (float)(e / 36.0);
+    const double q = e / 9.0;
+    g[1] = (float)q;
+    g[5] = (float)(0.25 * q);  // e / 36: the quotient by 9 times an exact power of two
+    g[7] = g[5];
 }
 
 // parabolic_D3Q19_x's node update (:456-530) on shifted populations: an opposite pair has one weight,

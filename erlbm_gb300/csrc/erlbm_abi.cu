@@ -100,6 +100,13 @@ struct erlbm_handle {
     // bc_graph_bc (rebuilt when a call brings other planes)
     cudaGraphExec_t bc_graph[2] = {nullptr, nullptr};
     BCp bc_graph_bc{};
+    bool bc_graph_by_three = false;
+    // three steps per launch with solids or planes (launch_d2q9_planes_x3), set up for the planes x3_planes
+    // by the first call that has steps enough; x3_state: 0 not tried, 1 ready, -1 not for these planes
+    int x3_state = 0, x3_planes[3] = {-1, -1, -1}, x3_listed[3] = {0, 0, 0};
+    uint8_t *d_x3_dist = nullptr;
+    int *d_x3_list = nullptr;
+    float *d_x3_mid = nullptr;
     cudaStream_t capture_stream = nullptr;
     size_t elem() const { return prec == ERLBM_FP32_SHIFTED ? sizeof(float) : 8; }  // FP64 or a float pair
 };
@@ -154,6 +161,9 @@ void free_handle(erlbm_handle *h)
     cudaFree(h->d_segflag);
     cudaFree(h->d_nodeflag);
     cudaFree(h->d_fix);
+    cudaFree(h->d_x3_dist);
+    cudaFree(h->d_x3_list);
+    cudaFree(h->d_x3_mid);
     cudaFree(h->d_profile);
     cudaFree(h->d_nof);
     cudaFree(h->d_buf[0]);
@@ -465,25 +475,73 @@ bool same_planes(const BCp &a, const BCp &b)
            a.profile == b.profile;
 }
 
-// A block of BC_GRAPH_STEPS steps of k_d2q9_hybrid as one CUDA graph launch, captured once per buffer
-// parity for the planes b.  The parabolic profile is read from h->d_profile when the graph runs, and
-// validate_bc rewrites it only after the stream has drained.
-constexpr int BC_GRAPH_STEPS = 64;
-
-int bc_graph_steps(erlbm_handle *h, const BCp &b)
+// Sets up three steps per launch for the planes b: node distances, the list of nodes that take the generic
+// update, the scratch buffer of the middle step.  Left to single steps (x3_state = -1) when more than a
+// quarter of the nodes would be listed or device memory is short.
+int setup_planes_x3(erlbm_handle *h, const BCp &b)
 {
-    if (!same_planes(h->bc_graph_bc, b)) {
+    const int planes[3] = {b.inlet_x, b.outlet_x, b.open_y};
+    CK(cudaStreamSynchronize(h->stream));  // steps in flight may read the lists of other planes
+    drop_bc_graphs(h);
+    memcpy(h->x3_planes, planes, sizeof(planes));
+    h->x3_state = -1;
+    cudaFree(h->d_x3_list);
+    h->d_x3_list = nullptr;
+    const size_t pop_bytes = (size_t)h->q * h->g.plane * sizeof(float);
+    if ((!h->d_x3_dist && cudaMalloc(&h->d_x3_dist, h->g.nbox) != cudaSuccess) ||
+        (!h->d_x3_mid && cudaMalloc(&h->d_x3_mid, pop_bytes) != cudaSuccess)) {
+        cudaGetLastError();
+        return ERLBM_OK;
+    }
+    uint8_t *fix = (uint8_t *)h->d_x3_mid;  // free until the first step
+    int *at = (int *)h->d_out, *n = h->x3_listed;
+    CK(cudaMemsetAsync(at, 0, 3 * sizeof(int), h->stream));
+    CKL(d2q9_fix_distance(h->g, b, fix, h->d_x3_dist, h->stream), "fix_distance");
+    CKL(d2q9_fix_list(h->g, fix, h->d_x3_dist, at, nullptr, h->stream), "fix_list");
+    CK(cudaMemcpyAsync(n, at, sizeof(h->x3_listed), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    const long long all = (long long)n[0] + n[1] + n[2];
+    if (all > h->g.nbox / 4) return ERLBM_OK;
+    if (cudaMalloc(&h->d_x3_list, (all > 0 ? all : 1) * sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();
+        h->d_x3_list = nullptr;
+        return ERLBM_OK;
+    }
+    const int from[3] = {0, n[0], n[0] + n[1]};
+    CK(cudaMemcpyAsync(at, from, sizeof(from), cudaMemcpyHostToDevice, h->stream));
+    CKL(d2q9_fix_list(h->g, fix, h->d_x3_dist, at, h->d_x3_list, h->stream), "fix_list");
+    h->x3_state = 1;
+    return ERLBM_OK;
+}
+
+int launch_planes_x3(const erlbm_handle *h, const BCp &b, int cur, cudaStream_t s)
+{
+    return launch_d2q9_planes_x3(h->op, h->g, b, h->R, (const float *)h->d_buf[cur], (float *)h->d_buf[cur ^ 1],
+                                 h->d_x3_mid, h->d_x3_dist, h->d_x3_list, h->x3_listed, s);
+}
+
+// A block of D2Q9 FP32 steps with solids or planes as one CUDA graph launch, captured once per buffer
+// parity for the planes b: 66 steps by threes, or 64 of k_d2q9_hybrid.  The parabolic profile is read from
+// h->d_profile when the graph runs, and validate_bc rewrites it only after the stream has drained.
+int bc_graph_steps_of(bool by_three) { return by_three ? 66 : 64; }
+
+int bc_graph_steps(erlbm_handle *h, const BCp &b, bool by_three)
+{
+    if (!same_planes(h->bc_graph_bc, b) || h->bc_graph_by_three != by_three) {
         drop_bc_graphs(h);
         h->bc_graph_bc = b;
+        h->bc_graph_by_three = by_three;
     }
     cudaGraphExec_t &x = h->bc_graph[h->cur];
     if (!x) {
         if (!h->capture_stream) CK(cudaStreamCreateWithFlags(&h->capture_stream, cudaStreamNonBlocking));
         CK(cudaStreamBeginCapture(h->capture_stream, cudaStreamCaptureModeRelaxed));
         int c = h->cur, lrc = 0;
-        for (int k = 0; k < BC_GRAPH_STEPS && lrc == 0; k++) {
-            lrc = launch_step_fp32_hybrid(h->op, h->g, b, h->R, (const float *)h->d_buf[c], (float *)h->d_buf[c ^ 1],
-                                          h->d_segflag, h->d_nodeflag, h->d_fix, h->n_fix, h->capture_stream);
+        for (int k = 0; k < bc_graph_steps_of(by_three) && lrc == 0; k += by_three ? 3 : 1) {
+            lrc = by_three ? launch_planes_x3(h, b, c, h->capture_stream)
+                           : launch_step_fp32_hybrid(h->op, h->g, b, h->R, (const float *)h->d_buf[c],
+                                                     (float *)h->d_buf[c ^ 1], h->d_segflag, h->d_nodeflag, h->d_fix,
+                                                     h->n_fix, h->capture_stream);
             c ^= 1;
         }
         cudaGraph_t graph = nullptr;
@@ -502,10 +560,13 @@ int bc_graph_steps(erlbm_handle *h, const BCp &b)
         }
     }
     CK(cudaGraphLaunch(x, h->stream));
-    h->steps_done += BC_GRAPH_STEPS;
+    h->steps_done += bc_graph_steps_of(by_three);
     h->kind = 1;
     return ERLBM_OK;
 }
+
+// Steps from which the set-up of three steps per launch with planes pays (@SETUP@).
+constexpr int X3_SETUP_STEPS = 48;
 
 // n_steps steps without checks, by graph blocks and multi-step launches where they apply.
 int advance(erlbm_handle *h, int n_steps, const BCp &b)
@@ -516,11 +577,29 @@ int advance(erlbm_handle *h, int n_steps, const BCp &b)
     PeriodicPlan p;
     if (plain) p = periodic_plan(h);
     const bool hybrid = fp32_2d && !plain && d2q9_hybrid_ok(h->g);
+    bool by_three = false;
+    if (fp32_2d && !plain && d2q9_planes_x3_ok(h->g)) {
+        auto current = [&] {
+            return h->x3_state != 0 && h->x3_planes[0] == b.inlet_x && h->x3_planes[1] == b.outlet_x &&
+                   h->x3_planes[2] == b.open_y;
+        };
+        // a call with few steps does not pay for the set-up
+        if (n_steps >= X3_SETUP_STEPS && !current())
+            if ((rc = setup_planes_x3(h, b))) return rc;
+        by_three = h->x3_state == 1 && current();
+    }
     for (int s = 0; s < n_steps;) {
         const int left = n_steps - s;
-        if (hybrid && h->kind == 1 && left >= BC_GRAPH_STEPS) {
-            if ((rc = bc_graph_steps(h, b))) return rc;
-            s += BC_GRAPH_STEPS;
+        if ((hybrid || by_three) && h->kind == 1 && left >= bc_graph_steps_of(by_three)) {
+            if ((rc = bc_graph_steps(h, b, by_three))) return rc;
+            s += bc_graph_steps_of(by_three);
+            continue;
+        }
+        if (by_three && h->kind == 1 && left >= 3) {
+            CKL(launch_planes_x3(h, b, h->cur, h->stream), "d2q9_planes_x3");
+            h->cur ^= 1;
+            h->steps_done += 3;
+            s += 3;
             continue;
         }
         if (plain && h->kind == 1 && (p.per_launch > 1 || p.fused1)) {

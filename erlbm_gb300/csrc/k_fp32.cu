@@ -276,12 +276,12 @@ __global__ void __launch_bounds__(128) k_periodic_d2q9_x2s(const float *__restri
         gather(g, bA, bB, nA, nB);  // output rows j, j + 1
         shifted::collide9x2<OP>(g, k);
         if (store) {
-            float *d0 = dst + (long long)j * nx + c, *d1 = d0 + nx;
-            const bool second = j + 1 < y1;  // an odd chunk's last iteration stores one row
+            // with an odd ny the last row pair is (ny - 1, ny): row ny is row 0, whose own warp stores the same bits
+            float *d0 = dst + (long long)j * nx + c, *d1 = dst + (long long)(j + 1 == ny ? 0 : j + 1) * nx + c;
 #pragma unroll
             for (int i = 0; i < 9; i++) {
                 d0[i * plane] = g[i].x;
-                if (second) d1[i * plane] = g[i].y;
+                d1[i * plane] = g[i].y;
             }
         }
 #pragma unroll
@@ -304,10 +304,15 @@ constexpr int X3_W = 28;
 
 // Four resident CTAs per SM: the register cap (128) spills 8 bytes, and 16 warps per SM instead of
 // 12 run 4 % faster on GB300 (158.6 against 151.9 G LU/s at L = 2048).
-template <int OP>
+// An odd ny: the last row pair is (ny - 1, ny), and row ny is row 0, whose own warp stores the same bits.
+// SKIP: nodes with dist[node] <= X3_SKIP are not stored (launch_d2q9_planes_x3).
+constexpr int X3_SKIP = 2;
+
+template <int OP, bool SKIP>
 __global__ void __launch_bounds__(128, 4) k_periodic_d2q9_x3s(const float *__restrict__ src, float *__restrict__ dst,
                                                           int nx, int ny, long long plane, int hc, int strips,
-                                                          int n_warps, shifted::Coef k)
+                                                          int n_warps, const uint8_t *__restrict__ dist,
+                                                          shifted::Coef k)
 {
     const int lane = threadIdx.x & 31;
     const int wid = (int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
@@ -447,12 +452,21 @@ __global__ void __launch_bounds__(128, 4) k_periodic_d2q9_x3s(const float *__res
         gather(g, cA, cB, mA, mB);  // output rows j, j + 1
         shifted::collide9x2<OP>(g, k);
         if (store) {
-            float *d0 = dst + (long long)j * nx + c, *d1 = d0 + nx;
-            const bool second = j + 1 < y1;  // an odd chunk's last iteration stores one row
+            const long long o0 = (long long)j * nx + c, o1 = (long long)(j + 1 == ny ? 0 : j + 1) * nx + c;
+            float *d0 = dst + o0, *d1 = dst + o1;
+            if (SKIP) {
+                const bool first = dist[o0] > X3_SKIP, second = dist[o1] > X3_SKIP;
 #pragma unroll
-            for (int i = 0; i < 9; i++) {
-                d0[i * plane] = g[i].x;
-                if (second) d1[i * plane] = g[i].y;
+                for (int i = 0; i < 9; i++) {
+                    if (first) d0[i * plane] = g[i].x;
+                    if (second) d1[i * plane] = g[i].y;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 9; i++) {
+                    d0[i * plane] = g[i].x;
+                    d1[i * plane] = g[i].y;
+                }
             }
         }
 #pragma unroll
@@ -517,10 +531,11 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-template <int OP, int MINB>
+template <int OP, int MINB, bool SKIP>
 __global__ void __launch_bounds__(128, MINB) k_periodic_d2q9_x3a(const float *__restrict__ src, float *__restrict__ dst,
                                                                 int nx, int ny, int plane, int hc, int strips,
-                                                                int n_warps, shifted::Coef k)
+                                                                int n_warps, const uint8_t *__restrict__ dist,
+                                                                shifted::Coef k)
 {
     extern __shared__ __align__(16) float xa_smem[];
     const int lane = threadIdx.x & 31;
@@ -588,6 +603,8 @@ __global__ void __launch_bounds__(128, MINB) k_periodic_d2q9_x3a(const float *__
         constexpr int t = decltype(T)::value % 3;
         constexpr int a = t, b = (t + 1) % 3, n = (t + 2) % 3;
         constexpr bool c1 = decltype(C1)::value, c2 = decltype(C2)::value;
+        uchar2 q = make_uchar2(255, 255);  // ahead of its use: the store is at the end of the iteration
+        if (SKIP && c2 && store && j < y1) q = *reinterpret_cast<const uchar2 *>(dist + (long long)j * nx + c);
         cp_async_wait<XA_DEPTH - 2>();
         __syncwarp();
         read(ring + ((t + 1) % 3) * XA_SLOT, g);
@@ -611,8 +628,16 @@ __global__ void __launch_bounds__(128, MINB) k_periodic_d2q9_x3a(const float *__
             if (s == 2) {
                 if (store && j < y1) {
                     float *d = dst + (long long)j * nx + c;
+                    if (!SKIP || (q.x > X3_SKIP && q.y > X3_SKIP)) {
 #pragma unroll
-                    for (int i = 0; i < 9; i++) *reinterpret_cast<float2 *>(d + (long long)i * plane) = g[i];
+                        for (int i = 0; i < 9; i++) *reinterpret_cast<float2 *>(d + (long long)i * plane) = g[i];
+                    } else if (q.x > X3_SKIP) {
+#pragma unroll
+                        for (int i = 0; i < 9; i++) d[(long long)i * plane] = g[i].x;
+                    } else if (q.y > X3_SKIP) {
+#pragma unroll
+                        for (int i = 0; i < 9; i++) d[(long long)i * plane + 1] = g[i].y;
+                    }
                 }
             } else {
                 s1[s][n][0] = g[3];
@@ -692,10 +717,11 @@ static void go_x2(const Geo &g, const shifted::Coef &k, const float *src, float 
 }
 
 // Three-step launch: as go_x2, over ceil(nx / 28) strips.
-template <int OP>
-static void go_x3(const Geo &g, const shifted::Coef &k, const float *src, float *dst, cudaStream_t s)
+template <int OP, bool SKIP = false>
+static void go_x3(const Geo &g, const shifted::Coef &k, const float *src, float *dst, cudaStream_t s,
+                  const uint8_t *dist = nullptr)
 {
-    auto kern = k_periodic_d2q9_x3s<OP>;
+    auto kern = k_periodic_d2q9_x3s<OP, SKIP>;
     constexpr int MAXDEV = 64;
     static std::atomic<int> warps_cache[MAXDEV];
     int dev = 0;
@@ -718,17 +744,18 @@ static void go_x3(const Geo &g, const shifted::Coef &k, const float *src, float 
     hc += hc & 1;
     if (hc > g.ny) hc = g.ny;
     const int n_warps = strips * (int)((g.ny + hc - 1) / hc);
-    kern<<<(unsigned)((n_warps + 3) / 4), 128, 0, s>>>(src, dst, g.nx, g.ny, g.plane, (int)hc, strips, n_warps, k);
+    kern<<<(unsigned)((n_warps + 3) / 4), 128, 0, s>>>(src, dst, g.nx, g.ny, g.plane, (int)hc, strips, n_warps, dist, k);
 }
 
 // Three-step launch over column pairs: ceil(nx / 60) strips, chunks of whole unrolled groups, as many
 // chunks per strip as one wave of resident warps holds (no second, partial wave).
 constexpr int XA_MINB = 4;  // resident 128-thread CTAs per SM (122 registers, no spills)
 
-template <int OP>
-static void go_x3a(const Geo &g, const shifted::Coef &k, const float *src, float *dst, cudaStream_t s)
+template <int OP, bool SKIP = false>
+static void go_x3a(const Geo &g, const shifted::Coef &k, const float *src, float *dst, cudaStream_t s,
+                   const uint8_t *dist = nullptr)
 {
-    auto kern = k_periodic_d2q9_x3a<OP, XA_MINB>;
+    auto kern = k_periodic_d2q9_x3a<OP, XA_MINB, SKIP>;
     const size_t smem = 4 * XA_SMEM_PER_WARP;
     constexpr int MAXDEV = 64;
     static std::atomic<int> warps_cache[MAXDEV];
@@ -751,15 +778,18 @@ static void go_x3a(const Geo &g, const shifted::Coef &k, const float *src, float
     if (hc < 2 * XP_SPAN) hc = 2 * XP_SPAN;
     const int n_warps = strips * (int)((g.ny + hc - 1) / hc);
     kern<<<(unsigned)((n_warps + 3) / 4), 128, smem, s>>>(src, dst, g.nx, g.ny, (int)g.plane, (int)hc, strips, n_warps,
-                                                         k);
+                                                         dist, k);
 }
 
-bool periodic_d2q9_x3a_ok(const Geo &g)
+// The 64-column strips' extent (with or without solids).
+static bool x3a_fits(const Geo &g)
 {
     // 64-column strips need ny >= 16; 16-byte copies start at multiples of four columns of any row; the nine
     // planes are addressed with 32-bit offsets
-    return g.solid == nullptr && g.nz == 1 && g.nx % 4 == 0 && g.ny >= 16 && g.nx >= 128 && 9 * g.plane < (1LL << 31);
+    return g.nz == 1 && g.nx % 4 == 0 && g.ny >= 16 && g.nx >= 128 && 9 * g.plane < (1LL << 31);
 }
+
+bool periodic_d2q9_x3a_ok(const Geo &g) { return g.solid == nullptr && x3a_fits(g); }
 
 // Rows per chunk of a three-step launch: one wave of `resident` warps covers the strips.
 static long long x3_rows(const Geo &g, long long resident, int width, int multiple, int least)
@@ -779,7 +809,7 @@ static long long x3_rows(const Geo &g, long long resident, int width, int multip
 // 76.5 / 87.2; the estimate picks the faster one in all of these (768^2, 4.35 / 4.79, it misses).
 bool periodic_d2q9_prefers_wide(const Geo &g)
 {
-    if (!periodic_d2q9_x3a_ok(g)) return false;
+    if (!x3a_fits(g)) return false;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -1110,6 +1140,182 @@ int launch_step_fp32_hybrid(int op, const Geo &g, const BCp &bc, const Relax &R,
     case OP_EXTREG:
         k_d2q9_hybrid<OP_EXTREG><<<(unsigned)nb, 256, 0, s>>>(src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb);
         break;
+    default: return -1;
+    }
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// ------------------------------------------------------------------------------------------------
+// Three steps per launch with solids and boundary planes
+// ------------------------------------------------------------------------------------------------
+
+namespace {
+
+constexpr int DIST_MAX = 4;  // distances counted; farther nodes hold DIST_MAX + 1
+
+// fix[node]: the fluid nodes that need the generic update: 1 next to a solid, 2 on a plane.
+__global__ void __launch_bounds__(256) k_fix_nodes(Geo g, int inlet_x, int outlet_x, int open_y, uint8_t *fix)
+{
+    const long long node = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (node >= g.nbox) return;
+    const int y = (int)(node / g.nx), x = (int)(node - (long long)y * g.nx);
+    uint8_t f = 0;
+    if (g.solid == nullptr || !g.solid[node]) {
+        if (g.solid != nullptr)
+            for (int dy = -1; dy <= 1; dy++)
+                for (int dx = -1; dx <= 1; dx++)
+                    f |= g.solid[(long long)wrap1(y + dy, g.ny) * g.nx + wrap1(x + dx, g.nx)] != 0;
+        if (x == inlet_x || x == outlet_x || y == open_y) f = 2;
+    }
+    fix[node] = f;
+}
+
+// dist[node]: Chebyshev distance (periodic) to the nearest such node, up to DIST_MAX.
+__global__ void __launch_bounds__(256) k_fix_distance(Geo g, const uint8_t *__restrict__ fix, uint8_t *dist)
+{
+    const long long node = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (node >= g.nbox) return;
+    const int y = (int)(node / g.nx), x = (int)(node - (long long)y * g.nx);
+    int d = DIST_MAX + 1;
+    for (int dy = -DIST_MAX; dy <= DIST_MAX; dy++) {
+        const uint8_t *row = fix + (long long)wrap1(y + dy, g.ny) * g.nx;
+        for (int dx = -DIST_MAX; dx <= DIST_MAX; dx++)
+            if (row[wrap1(x + dx, g.nx)]) d = min(d, max(abs(dx), abs(dy)));
+    }
+    dist[node] = (uint8_t)d;
+}
+
+// Lists the fluid nodes within DIST_MAX that lie on no plane, in three groups: distance <= 2, 3, 4.  at[k]:
+// where group k goes on (counted only while list is null).
+__global__ void __launch_bounds__(256) k_fix_list(Geo g, const uint8_t *__restrict__ fix,
+                                                  const uint8_t *__restrict__ dist, int *at, int *list)
+{
+    const long long node = (long long)blockIdx.x * 256 + threadIdx.x;
+    int group = -1;
+    if (node < g.nbox) {
+        const int d = dist[node];
+        if (d <= DIST_MAX && fix[node] != 2 && (g.solid == nullptr || !g.solid[node])) group = d <= X3_SKIP ? 0 : d - X3_SKIP;
+    }
+    const int lane = threadIdx.x & 31;
+    for (int k = 0; k < 3; k++) {
+        const unsigned m = __ballot_sync(FULL, group == k);
+        if (m == 0) continue;
+        int base = 0;
+        if (lane == 0) base = atomicAdd(at + k, __popc(m));
+        base = __shfl_sync(FULL, base, 0);
+        if (group == k && list != nullptr) list[base + __popc(m & ((1u << lane) - 1))] = (int)node;
+    }
+}
+
+// One generic step at the nodes of the planes and the first n_list listed ones.  Bound by latency (list entry,
+// populations, collision, and on a plane its FP64 closure: about 75 cycles per dependent FP64 operation), so
+// the plane nodes have warps of their own: among the others, in row order, one of them would hold up a
+// warp per row (9.2 -> @LS@ us per launch on the 4096 x 1024 channel).
+template <int OP>
+__global__ void __launch_bounds__(64) k_listed_step(const float *__restrict__ src, float *__restrict__ dst, Geo g,
+                                                    BCp bc, shifted::Coef k, const int *__restrict__ list, int n_list,
+                                                    int n_planes)
+{
+    int t = (int)(blockIdx.x * 64 + threadIdx.x);
+    int x, y, node;
+    float f[9];
+    if (t >= n_planes) {  // n_planes is a multiple of 32
+        t -= n_planes;
+        if (t >= n_list) return;
+        node = list[t];
+        y = node / g.nx;
+        x = node - y * g.nx;
+        gather<PrecShifted32, 9>(src, g, 0, x, y, 0, node, f);
+    } else {
+        if (bc.inlet_x >= 0) {
+            if (t < g.ny) { x = bc.inlet_x; y = t; goto have; }
+            t -= g.ny;
+        }
+        if (bc.outlet_x >= 0) {
+            if (t < g.ny) { x = bc.outlet_x; y = t; goto have; }
+            t -= g.ny;
+        }
+        if (bc.open_y < 0 || t >= g.nx) return;
+        x = t;
+        y = bc.open_y;
+    have:
+        node = y * g.nx + x;
+        if (g.solid != nullptr && g.solid[node]) return;
+        state_after_planes<PrecShifted32, 9>(src, g, bc, 0, x, y, 0, node, f);
+    }
+    shifted::collide<9, OP>(f, k);
+#pragma unroll
+    for (int i = 0; i < 9; i++) dst[(long long)i * g.plane + node] = f[i];
+}
+
+template <int OP>
+void go_planes_x3(const Geo &g, const BCp &bc, const shifted::Coef &k, const float *src, float *dst, float *mid,
+                  const uint8_t *dist, const int *list, const int n[3], bool wide, cudaStream_t s)
+{
+    const int planes = ((bc.inlet_x >= 0 ? g.ny : 0) + (bc.outlet_x >= 0 ? g.ny : 0) + (bc.open_y >= 0 ? g.nx : 0) + 31) / 32 * 32;
+    auto listed = [&](const float *from, float *to, int count) {
+        if (planes + count > 0)
+            k_listed_step<OP><<<(unsigned)((planes + count + 63) / 64), 64, 0, s>>>(from, to, g, bc, k, list, count,
+                                                                                   planes);
+    };
+    listed(src, dst, n[0] + n[1] + n[2]);
+    listed(dst, mid, n[0] + n[1]);
+    listed(mid, dst, n[0]);
+    if (wide)
+        go_x3a<OP, true>(g, k, src, dst, s, dist);
+    else
+        go_x3<OP, true>(g, k, src, dst, s, dist);
+}
+
+}  // namespace
+
+// From the sizes on where three steps by threes beat three single steps: a launch sequence costs three
+// latency-bound listed launches (about 5 us each), whatever the size, and saves two thirds of the traffic, or, where
+// nx % 128 != 0, the generic per-node kernel.  Measured on channels, us per step, single against threes:
+// @RULE@
+bool d2q9_planes_x3_ok(const Geo &g)
+{
+    return g.nz == 1 && g.nx >= 32 && g.ny >= 16 && g.nbox < (1LL << 31) - 256 &&
+           g.nbox >= (d2q9_hybrid_ok(g) ? 1500000 : 200000);
+}
+
+int d2q9_fix_distance(const Geo &g, const BCp &bc, uint8_t *fix, uint8_t *dist, cudaStream_t s)
+{
+    const unsigned nb = blocks_for(g.nbox, 256);
+    k_fix_nodes<<<nb, 256, 0, s>>>(g, bc.inlet_x, bc.outlet_x, bc.open_y, fix);
+    k_fix_distance<<<nb, 256, 0, s>>>(g, fix, dist);
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+int d2q9_fix_list(const Geo &g, const uint8_t *fix, const uint8_t *dist, int *at, int *list, cudaStream_t s)
+{
+    k_fix_list<<<blocks_for(g.nbox, 256), 256, 0, s>>>(g, fix, dist, at, list);
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+// Three steps of a D2Q9 box with solids or planes (d2q9_planes_x3_ok).  The strips of the periodic
+// three-step kernels are right wherever no generic node (next to a solid, on a plane) is within two steps'
+// reach: the nodes farther than X3_SKIP = 2 from one, which is what they store.  The nodes within 2 are taken
+// through the three steps one by one with the generic update: step one at distance <= 4 into dst (not
+// yet written by the strips), step two at distance <= 3 from there into mid, step three at distance <= 2 from mid
+// into dst.  A generic update reads its neighbours, and on a plane its inner neighbour's neighbours, so each
+// step's nodes find what they pull among the step before's: distance 3 pulls from 4, distance 2 from 3, a plane node
+// (distance 0) from 2 at most.  The strips also compute the nodes they skip, and solid nodes, from
+// populations that are not theirs; nothing they store depends on those.  Every stored value is the generic
+// kernel's, bit for bit.
+// HBM bytes per update drop from 72 to 24 plus the listed nodes': 4096 x 1024 with walls, a cylinder and two
+// planes (@LIST@ listed nodes): @CH0@ us per three steps in single steps -> @CH1@ us.
+int launch_d2q9_planes_x3(int op, const Geo &g, const BCp &bc, const Relax &R, const float *src, float *dst, float *mid,
+                          const uint8_t *dist, const int *list, const int n[3], cudaStream_t s)
+{
+    if (!d2q9_planes_x3_ok(g)) return -1;
+    const shifted::Coef k = shifted::make_coef(R);
+    const bool wide = periodic_d2q9_prefers_wide(g);
+    switch (op) {
+    case OP_BGK: go_planes_x3<OP_BGK>(g, bc, k, src, dst, mid, dist, list, n, wide, s); break;
+    case OP_MRT: go_planes_x3<OP_MRT>(g, bc, k, src, dst, mid, dist, list, n, wide, s); break;
+    case OP_REG: go_planes_x3<OP_REG>(g, bc, k, src, dst, mid, dist, list, n, wide, s); break;
+    case OP_EXTREG: go_planes_x3<OP_EXTREG>(g, bc, k, src, dst, mid, dist, list, n, wide, s); break;
     default: return -1;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -3;

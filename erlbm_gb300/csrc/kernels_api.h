@@ -75,6 +75,16 @@ bool periodic_d2q9_prefers_wide(const Geo &g);
 bool periodic_d3q19_fp32_ok(const Geo &g);
 int launch_periodic_d3q19_fp32(int op, const Geo &g, const Relax &R, const float *src, float *dst, cudaStream_t s);
 
+// Three steps per launch sequence of a D2Q9 FP32-shifted box with solids or planes.  d2q9_fix_distance fills
+// dist (a byte per node) and fix (the same, needed for d2q9_fix_list); d2q9_fix_list adds the sizes of the
+// three groups of listed nodes to at (list = null), or lists them from the offsets in at on.  n: the group
+// sizes.  mid: scratch, one population buffer.
+bool d2q9_planes_x3_ok(const Geo &g);
+int d2q9_fix_distance(const Geo &g, const BCp &bc, uint8_t *fix, uint8_t *dist, cudaStream_t s);
+int d2q9_fix_list(const Geo &g, const uint8_t *fix, const uint8_t *dist, int *at, int *list, cudaStream_t s);
+int launch_d2q9_planes_x3(int op, const Geo &g, const BCp &bc, const Relax &R, const float *src, float *dst, float *mid,
+                          const uint8_t *dist, const int *list, const int n[3], cudaStream_t s);
+
 // Stream only: dst = post-stream populations of the post-collision state src (no BC, no collision).
 int launch_stream_only_fp64(int q, const Geo &g, const double *src, double *dst, cudaStream_t s);
 int launch_stream_only_fp32(int q, const Geo &g, const float *src, float *dst, cudaStream_t s);

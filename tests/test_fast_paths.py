@@ -88,3 +88,39 @@ def test_run_without_density_checks_takes_the_stepping_path():
         b.step(250)
         assert r["label"] == 0 and r["steps_done"] == 250
         assert np.array_equal(a.get_populations(), b.get_populations())
+
+
+@pytest.mark.parametrize("nx,ny,op", [(1000, 250, 4), (1003, 211, 3), (701, 300, 2), (1536, 1024, 4), (1660, 922, 1)])
+@pytest.mark.parametrize("planes", ["channel", "open", "density", "solids"])
+def test_three_steps_per_launch_with_planes_equal_single_steps(nx, ny, op, planes):
+    """Boxes with walls, an obstacle, scattered solids (also on the seams) and boundary planes take three steps per
+    launch in calls of many steps; calls of one step run one at a time.  The same bits, through graph blocks, single
+    launches and leftover steps."""
+    import erlbm_gb300 as E
+    rng = np.random.default_rng(nx + ny)
+    s = np.zeros((ny, nx), np.uint8)
+    if planes in ("channel", "density"):
+        s[0] = s[-1] = s[:, 0] = s[:, -1] = 1
+    if planes != "open":
+        y, x = np.mgrid[0:ny, 0:nx]
+        s[(x - nx // 3) ** 2 + (y - ny // 2) ** 2 <= (ny // 10) ** 2] = 1
+        s[rng.integers(0, ny, 30), rng.integers(0, nx, 30)] = 1
+        s[ny // 2, nx - 1] = s[0, nx // 2] = 1
+    bc = {"channel": dict(inlet_x=1, inlet_kind=E.INLET_PARABOLIC, parabolic_L=ny - 2, u_in=0.05, outlet_x=nx - 2,
+                          outlet_kind=E.OUTLET_CONVECTIVE),
+          "density": dict(inlet_x=1, u_in=0.04, outlet_x=nx - 2),
+          "open": dict(inlet_x=0, u_in=0.03, outlet_x=nx - 1, outlet_kind=E.OUTLET_OPEN, open_y=ny - 1),
+          "solids": None}[planes]
+    with E.Lattice(9, nx, ny, 1, s.reshape(-1) if s.any() else None, 0.55, 1.0 if op == 3 else 0.7, op,
+                   E.FP32_SHIFTED) as a, \
+            E.Lattice(9, nx, ny, 1, s.reshape(-1) if s.any() else None, 0.55, 1.0 if op == 3 else 0.7, op,
+                      E.FP32_SHIFTED) as b:
+        w = np.array([4 / 9] + [1 / 9] * 4 + [1 / 36] * 4)
+        f = (w[None, :] * (1.0 + 0.03 * rng.standard_normal((a.n_fluid, 9)))).ravel()
+        a.set_populations(f)
+        b.set_populations(f)
+        a.step(72, bc)
+        for _ in range(72):
+            b.step(1, bc)
+        assert np.array_equal(a.get_populations(E.STAGE_POST_COLLISION), b.get_populations(E.STAGE_POST_COLLISION))
+        assert np.array_equal(a.get_populations(), b.get_populations())
