@@ -33,6 +33,7 @@
 // D2Q9 E-RLBM: 169 -> 160 operations per update.
 #pragma once
 
+#include "fp64_int.cuh"
 #include "lattice.cuh"
 
 namespace erlbm {
@@ -89,6 +90,36 @@ __device__ __forceinline__ void equilibrium9(double rho, double ux, double uy, d
     feq_pair(uy, yy, wr1, C, feq[3], feq[4]);
     feq_pair(sp, sp * sp, wr2, C, feq[5], feq[6]);
     feq_pair(sm, sm * sm, wr2, C, feq[7], feq[8]);
+}
+
+// The same for the collision: where the velocity is below the bound of fp64int::eq_pair (Mach 0.28) the sums of
+// the pairs' polynomials run on the integer pipes, nine FP64 operations less per pair.
+__device__ __forceinline__ uint32_t abs_hi(double x) { return (uint32_t)__double2hiint(x) & 0x7fffffffu; }
+
+__device__ __forceinline__ void feq_pair_int(double cv, double cv2, double wr, uint64_t C62, double &fa, double &fb)
+{
+    double a, b;
+    fp64int::eq_pair(cv, cv2, C62, a, b);
+    fa = wr * a;
+    fb = wr * b;
+}
+
+__device__ __forceinline__ void equilibrium9_int(double rho, double ux, double uy, double feq[9])
+{
+    const double sp = ux + uy, sm = ux - uy;
+    if (max(abs_hi(sp), abs_hi(sm)) >= fp64int::EQ_MAX_HI) {  // |ux|, |uy| <= max(|sp|, |sm|)
+        equilibrium9(rho, ux, uy, feq);
+        return;
+    }
+    const double xx = ux * ux, yy = uy * uy;
+    const double C = 1.5 * (xx + yy);
+    const uint64_t C62 = fp64int::fixed62(C);
+    const double wr1 = (1. / 9.) * rho, wr2 = (1. / 36.) * rho;
+    feq[0] = ((4. / 9.) * rho) * (1.0 - C);
+    feq_pair_int(ux, xx, wr1, C62, feq[1], feq[2]);
+    feq_pair_int(uy, yy, wr1, C62, feq[3], feq[4]);
+    feq_pair_int(sp, sp * sp, wr2, C62, feq[5], feq[6]);
+    feq_pair_int(sm, sm * sm, wr2, C62, feq[7], feq[8]);
 }
 
 // Row ROW of the MRT transform applied to f: the reference sums M[ROW][i] * f[i] from 0.0 in
@@ -158,12 +189,28 @@ __device__ __forceinline__ void collide9_mrt(double f[9], const Relax &R, const 
     f[8] = mrt9_back<8>(m);
 }
 
+// Whether every sum of up to 2^M of the d_i = f_i - feq_i, i >= 1, is exact in any order: all of them are multiples
+// of the last place 2^(e-52) of the smallest f_i or feq_i (exponent e), and with every |d_i| < 2^(e-M+1) no sum
+// exceeds 2^53 of those.  Then the terms that the sums of d share are added once.
+template <int Q, int M>
+__device__ __forceinline__ bool exact_sums(const double *f, const double *feq, const double *d)
+{
+    int least = __double2hiint(f[1]);  // negative for a negative value
+    unsigned most = 0;
+#pragma unroll
+    for (int i = 1; i < Q; i++) {
+        least = min(least, min(__double2hiint(f[i]), __double2hiint(feq[i])));
+        most = max(most, abs_hi(d[i]));
+    }
+    return (int)(most >> 20) + M <= (least >> 20);
+}
+
 template <int OP>
 __device__ __forceinline__ void collide9(double f[9], const Relax &R)
 {
     double rho, ux, uy, feq[9];
     moments9(f, rho, ux, uy);
-    equilibrium9(rho, ux, uy, feq);
+    equilibrium9_int(rho, ux, uy, feq);
     if constexpr (OP == OP_MRT) {
         collide9_mrt(f, R, feq);
         return;
@@ -176,9 +223,17 @@ __device__ __forceinline__ void collide9(double f[9], const Relax &R)
     double d[9];
 #pragma unroll
     for (int i = 0; i < 9; i++) d[i] = f[i] - feq[i];
-    const double pxx = ((((d[1] + d[2]) + d[5]) + d[6]) + d[7]) + d[8];
-    const double pyy = ((((d[3] + d[4]) + d[5]) + d[6]) + d[7]) + d[8];
-    const double pxy = ((d[5] + d[6]) - d[7]) - d[8];
+    double pxx, pyy, pxy;
+    if (exact_sums<9, 3>(f, feq, d)) {
+        const double s56 = d[5] + d[6], s78 = d[7] + d[8], t = s56 + s78;
+        pxx = (d[1] + d[2]) + t;
+        pyy = (d[3] + d[4]) + t;
+        pxy = s56 - s78;
+    } else {
+        pxx = ((((d[1] + d[2]) + d[5]) + d[6]) + d[7]) + d[8];
+        pyy = ((((d[3] + d[4]) + d[5]) + d[6]) + d[7]) + d[8];
+        pxy = ((d[5] + d[6]) - d[7]) - d[8];
+    }
     const double xa = QA * pxx, xb = QB * pxx, ya = QA * pyy, yb = QB * pyy;
     const double dd = xa + ya;
     double f1[9];
@@ -243,12 +298,37 @@ __device__ __forceinline__ void equilibrium19(double rho, double ux, double uy, 
     feq_pair(zmy, zmy * zmy, wr2, C, feq[17], feq[18]);
 }
 
+__device__ __forceinline__ void equilibrium19_int(double rho, double ux, double uy, double uz, double feq[19])
+{
+    const double xpy = ux + uy, xmy = ux - uy, xpz = ux + uz, xmz = ux - uz, ypz = uy + uz, zmy = uz - uy;
+    const uint32_t most = max(max(max(abs_hi(xpy), abs_hi(xmy)), max(abs_hi(xpz), abs_hi(xmz))),
+                              max(abs_hi(ypz), abs_hi(zmy)));
+    if (most >= fp64int::EQ_MAX_HI) {
+        equilibrium19(rho, ux, uy, uz, feq);
+        return;
+    }
+    const double xx = ux * ux, yy = uy * uy, zz = uz * uz;
+    const double C = 1.5 * ((xx + yy) + zz);
+    const uint64_t C62 = fp64int::fixed62(C);
+    const double wr1 = (1. / 18.) * rho, wr2 = (1. / 36.) * rho;
+    feq[0] = ((1. / 3.) * rho) * (1.0 - C);
+    feq_pair_int(ux, xx, wr1, C62, feq[1], feq[2]);
+    feq_pair_int(uy, yy, wr1, C62, feq[3], feq[4]);
+    feq_pair_int(uz, zz, wr1, C62, feq[5], feq[6]);
+    feq_pair_int(xpy, xpy * xpy, wr2, C62, feq[7], feq[8]);
+    feq_pair_int(xmy, xmy * xmy, wr2, C62, feq[9], feq[10]);
+    feq_pair_int(xpz, xpz * xpz, wr2, C62, feq[11], feq[12]);
+    feq_pair_int(xmz, xmz * xmz, wr2, C62, feq[13], feq[14]);
+    feq_pair_int(ypz, ypz * ypz, wr2, C62, feq[16], feq[15]);
+    feq_pair_int(zmy, zmy * zmy, wr2, C62, feq[17], feq[18]);
+}
+
 template <int OP>
 __device__ __forceinline__ void collide19(double f[19], const Relax &R)
 {
     double rho, ux, uy, uz, feq[19];
     moments19(f, rho, ux, uy, uz);
-    equilibrium19(rho, ux, uy, uz, feq);
+    equilibrium19_int(rho, ux, uy, uz, feq);
     if (OP == OP_BGK) {
 #pragma unroll
         for (int i = 0; i < 19; i++) f[i] = f[i] + (feq[i] - f[i]) * R.inv_tau;
@@ -257,12 +337,25 @@ __device__ __forceinline__ void collide19(double f[19], const Relax &R)
     double d[19];
 #pragma unroll
     for (int i = 0; i < 19; i++) d[i] = f[i] - feq[i];
-    const double pxx = ((((((((d[1] + d[2]) + d[7]) + d[8]) + d[9]) + d[10]) + d[11]) + d[12]) + d[13]) + d[14];
-    const double pyy = ((((((((d[3] + d[4]) + d[7]) + d[8]) + d[9]) + d[10]) + d[15]) + d[16]) + d[17]) + d[18];
-    const double pzz = ((((((((d[5] + d[6]) + d[11]) + d[12]) + d[13]) + d[14]) + d[15]) + d[16]) + d[17]) + d[18];
-    const double pxy = ((d[7] + d[8]) - d[9]) - d[10];
-    const double pxz = ((d[11] + d[12]) - d[13]) - d[14];
-    const double pyz = ((d[15] + d[16]) - d[17]) - d[18];
+    double pxx, pyy, pzz, pxy, pxz, pyz;
+    if (exact_sums<19, 4>(f, feq, d)) {
+        const double a = d[7] + d[8], b = d[9] + d[10], ab = a + b;
+        const double g = d[11] + d[12], h = d[13] + d[14], gh = g + h;
+        const double m = d[15] + d[16], n = d[17] + d[18], mn = m + n;
+        pxx = (d[1] + d[2]) + (ab + gh);
+        pyy = (d[3] + d[4]) + (ab + mn);
+        pzz = (d[5] + d[6]) + (gh + mn);
+        pxy = a - b;
+        pxz = g - h;
+        pyz = m - n;
+    } else {
+        pxx = ((((((((d[1] + d[2]) + d[7]) + d[8]) + d[9]) + d[10]) + d[11]) + d[12]) + d[13]) + d[14];
+        pyy = ((((((((d[3] + d[4]) + d[7]) + d[8]) + d[9]) + d[10]) + d[15]) + d[16]) + d[17]) + d[18];
+        pzz = ((((((((d[5] + d[6]) + d[11]) + d[12]) + d[13]) + d[14]) + d[15]) + d[16]) + d[17]) + d[18];
+        pxy = ((d[7] + d[8]) - d[9]) - d[10];
+        pxz = ((d[11] + d[12]) - d[13]) - d[14];
+        pyz = ((d[15] + d[16]) - d[17]) - d[18];
+    }
     const double xa = QA * pxx, xb = QB * pxx;
     const double ya = QA * pyy, yb = QB * pyy;
     const double za = QA * pzz, zb = QB * pzz;

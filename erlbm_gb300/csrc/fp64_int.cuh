@@ -1,0 +1,110 @@
+// fp64_int.cuh -- parts of the exact FP64 collision on the integer pipes, with the FP64 pipe's bits.
+//
+// GB300 issues two FP64 operations per clock and SM (a warp instruction holds its scheduler's FP64 pipe for 64
+// cycles), but 64 integer ALU operations and 64 integer multiply-adds.  Where the range of the operands is known,
+// a correctly rounded FP64 add is an integer add and a rounding to a fixed bit position, about a dozen integer
+// instructions, and runs beside the FP64 work of the other warps.  Everything here is integer arithmetic from the
+// definition of round-to-nearest-even; the results are the IEEE ones, bit for bit.
+#pragma once
+
+#include <cstdint>
+
+namespace erlbm {
+namespace fp64int {
+
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ uint64_t bits(double x) { return (uint64_t)__double_as_longlong(x); }
+__device__ __forceinline__ double from_bits(uint64_t b) { return __longlong_as_double((long long)b); }
+#else
+inline uint64_t bits(double x)
+{
+    uint64_t b;
+    __builtin_memcpy(&b, &x, 8);
+    return b;
+}
+inline double from_bits(uint64_t b)
+{
+    double x;
+    __builtin_memcpy(&x, &b, 8);
+    return x;
+}
+#endif
+
+__host__ __device__ __forceinline__ uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
+__host__ __device__ __forceinline__ uint64_t mantissa(uint64_t b) { return (b & 0xfffffffffffffull) | 0x10000000000000ull; }
+__host__ __device__ __forceinline__ int exponent(uint64_t b) { return (int)(hi32(b) >> 20) & 0x7ff; }
+
+// x rounded to a multiple of 2^K, ties to even.
+template <int K>
+__host__ __device__ __forceinline__ uint64_t round_at(uint64_t x)
+{
+    const uint64_t r = x + ((1u << (K - 1)) - 1) + ((uint32_t)x >> K & 1u);
+    return r & ~(uint64_t)((1u << K) - 1);
+}
+// The same at bit k (k < 32).
+__host__ __device__ __forceinline__ uint64_t round_at(uint64_t x, int k)
+{
+    const uint32_t low = 1u << k;
+    const uint64_t r = x + ((low >> 1) - 1) + ((uint32_t)x >> k & 1u);
+    return r & ~(uint64_t)(low - 1);
+}
+
+// x >> sh (0 <= sh <= 63) with a 1 in the last place if a bit was lost: enough for any later rounding at a
+// higher place to go the way the exact value would.
+__host__ __device__ __forceinline__ uint64_t shift_sticky(uint64_t x, int sh)
+{
+    const uint64_t t = x >> sh;
+    return t | (uint64_t)((t << sh) != x);
+}
+
+constexpr uint64_t ONE62 = 1ull << 62;
+
+// A double 0 <= x < 1 in units of 2^-62, lost bits sticky (0 gives 0 or 1: see eq_pair).
+__host__ __device__ __forceinline__ uint64_t fixed62(double x)
+{
+    const uint64_t b = bits(x);
+    const int sh = 1022 - exponent(b);
+    return shift_sticky(mantissa(b) << 9, sh < 63 ? sh : 63);
+}
+
+// The velocity components and their sums eq_pair takes are below this in modulus.
+constexpr double EQ_MAX = 0.16;
+constexpr uint32_t EQ_MAX_HI = 0x3fc47ae1u;  // upper word of 0.16
+
+// ((1 + t) + B) - C and ((1 - t) + B) - C with t = RN(3 cv), B = RN(3 RN(1.5 cv2)), every sum rounded, for |cv| <
+// EQ_MAX, cv2 = RN(cv cv) and C = RN(1.5 u^2) in the form of fixed62, C < 0.12.  In units of 2^-62, sums below
+// 1 are rounded at bit 9 and sums in [1, 2) at bit 10.  With a = |t| <= 0.48, 1 + a and (1 + a) + B lie in [1, 2);
+// 1 - a, (1 - a) + B (B <= 0.24 |t|) and that less C lie in [1/2, 1]; only (1 + a) + B less C can lie on either
+// side of 1.  A sum that rounds up to 1 at bit 9 is 1.  Zero operands come out of the shifts as 0 or sticky 1, and
+// one unit more or less beside a multiple of 2^9 does not change a rounding.  Nine FP64 operations.
+__host__ __device__ __forceinline__ void eq_pair(double cv, double cv2, uint64_t C62, double &plus, double &minus)
+{
+    const uint64_t bc = bits(cv), bp = bits(cv2);
+    // t: 3 m has 54 or 55 bits, rounded to 53; 2^7 (3 m) 2^(E - 1020) is t in units of 2^-62
+    const uint64_t m3 = mantissa(bc) * 3u;
+    const uint64_t v = round_at(m3, 1 + (int)(hi32(m3) >> 22));
+    const int st = 1020 - exponent(bc);
+    const uint64_t t = shift_sticky(v << 7, st < 63 ? st : 63);
+    // B: the same twice; 3 times the first has 56 or 57 bits
+    const uint64_t n3 = mantissa(bp) * 3u;
+    const uint64_t n9 = round_at(n3, 1 + (int)(hi32(n3) >> 22)) * 3u;
+    const uint64_t w = round_at(n9, 3 + (int)(hi32(n9) >> 24));
+    const int sb = 1019 - exponent(bp);
+    const uint64_t B = shift_sticky(w << 5, sb < 63 ? sb : 63);
+
+    uint64_t p = round_at<10>(ONE62 + t), q = round_at<9>(ONE62 - t);
+    p = round_at<10>(p + B);
+    q = round_at<9>(q + B);
+    p = p - C62;
+    const int k = 9 + (int)(hi32(p) >> 30);
+    p = round_at(p, k);
+    q = round_at<9>(q - C62);
+    // units of 2^-62 to a double: the leading bit adds 1 to the exponent field
+    const uint64_t up = (p >> k) + ((uint64_t)(1012 + k) << 52), uq = (q >> 9) + (1021ull << 52);
+    const bool neg = (int64_t)bc < 0;
+    plus = from_bits(neg ? uq : up);
+    minus = from_bits(neg ? up : uq);
+}
+
+}  // namespace fp64int
+}  // namespace erlbm

@@ -1,0 +1,49 @@
+// Compares the integer forms of erlbm_gb300/csrc/fp64_int.cuh with the FP64 operations they stand for, on the CPU.
+// Prints "cases bad" (build with -ffp-contract=off).
+#define __host__
+#define __device__
+#define __forceinline__ inline
+#include "../../erlbm_gb300/csrc/fp64_int.cuh"
+
+#include <cmath>
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+
+using namespace erlbm::fp64int;
+
+static std::mt19937_64 rng;
+
+// A value of modulus below `most`: any scale down to underflow, short mantissas (ties), zeros of both signs.
+static double draw(double most)
+{
+    const double x = std::ldexp((double)(int64_t)rng(), -63) * most;
+    switch (rng() % 8) {
+    case 0: return std::ldexp(x, -(int)(rng() % 70));
+    case 1: return std::ldexp(x, -(int)(rng() % 1100));
+    case 2: return std::ldexp((double)((int)(rng() % 33) - 16), -8 - (int)(rng() % 6)) * (most / 0.08);
+    case 3: return rng() % 4 ? x : 0.0 * x;
+    default: return std::ldexp(x, -(int)(rng() % 8));
+    }
+}
+
+int main(int argc, char **argv)
+{
+    rng.seed(7);
+    const long n = argc > 1 ? atol(argv[1]) : 1000000;
+    long cases = 0, bad = 0;
+    for (long it = 0; it < n; it++) {
+        const double u[3] = {draw(0.08), draw(0.08), draw(0.08)};
+        const double cv = it % 4 == 0 ? u[0] : it % 4 == 1 ? u[0] + u[1] : it % 4 == 2 ? u[0] - u[1] : 2.0 * u[0];
+        const double C = 1.5 * ((u[0] * u[0] + u[1] * u[1]) + u[2] * u[2]);
+        if (!(std::fabs(cv) < EQ_MAX) || !(C < 0.115)) continue;
+        const double t3 = cv * 3., B = ((0.5 * cv) * cv * 3.) * 3.;
+        const double a = ((1.0 + t3) + B) - C, b = ((1.0 - t3) + B) - C;
+        double p, m;
+        eq_pair(cv, cv * cv, fixed62(C), p, m);
+        cases++;
+        bad += bits(p) != bits(a) || bits(m) != bits(b);
+    }
+    printf("%ld %ld\n", cases, bad);
+    return 0;
+}
