@@ -498,9 +498,8 @@ __device__ BatchResult batch_one_run(const BatchGeo &g, const BatchRun &r, const
     return o;
 }
 
-template <class P, int Q, int NPT>
-__global__ void __launch_bounds__(BatchBounds<NPT, sizeof(typename P::T)>::MAXT,
-                                  BatchBounds<NPT, sizeof(typename P::T)>::MINB)
+template <class P, int Q, int NPT, int MAXT = BatchBounds<NPT, sizeof(typename P::T)>::MAXT>
+__global__ void __launch_bounds__(MAXT, BatchBounds<NPT, sizeof(typename P::T)>::MINB)
     k_batch(BatchGeo g, const BatchRun *__restrict__ runs, int n_runs, int *__restrict__ counter,
             BatchResult *__restrict__ res, const double *__restrict__ aos, int dbl)
 {

@@ -122,6 +122,51 @@ __device__ __forceinline__ void equilibrium9_int(double rho, double ux, double u
     feq_pair_int(sm, sm * sm, wr2, C62, feq[7], feq[8]);
 }
 
+// Whether all Q populations have the fixed-point form of fp64int.
+template <int Q>
+__device__ __forceinline__ bool fixed_form(const double *f)
+{
+    uint32_t most = 0;
+#pragma unroll
+    for (int i = 0; i < Q; i++) most = max(most, fp64int::fix_range(f[i]));
+    return most < fp64int::FIX_SPAN;
+}
+
+// moments9 with its sums in fixed point (fixed_form holds), every partial sum rounded as the FP64 add rounds it:
+// 18 FP64 operations less.  F: the populations in fixed point.
+__device__ __forceinline__ void moments9_fixed(const double f[9], int64_t F[9], double &rho, double &ux, double &uy)
+{
+    using fp64int::round53;
+#pragma unroll
+    for (int i = 0; i < 9; i++) F[i] = fp64int::to_fixed(f[i]);
+    int64_t r = F[0];
+#pragma unroll
+    for (int i = 1; i < 9; i++) r = round53(r + F[i]);
+    int64_t mx = round53(F[1] - F[2]), my = round53(F[3] - F[4]);
+    mx = round53(round53(round53(round53(mx + F[5]) - F[6]) + F[7]) - F[8]);
+    my = round53(round53(round53(round53(my + F[5]) - F[6]) - F[7]) + F[8]);
+    rho = fp64int::to_double(r);
+    const double inv = 1.0 / rho;
+    ux = fp64int::to_double(mx) * inv;
+    uy = fp64int::to_double(my) * inv;
+}
+
+// D_i = f_i - feq_i in fixed point.  True when every feq has the fixed-point form too and every |D_i| < 2^(53 - M):
+// then each D_i is exact, and so is every sum of up to 2^M of them in any order.
+template <int Q, int M>
+__device__ __forceinline__ bool fixed_parts(const int64_t *F, const double *feq, int64_t *D)
+{
+    if (!fixed_form<Q>(feq)) return false;
+    uint32_t most = 0;
+#pragma unroll
+    for (int i = 0; i < Q; i++) {
+        D[i] = F[i] - fp64int::to_fixed(feq[i]);
+        const int32_t h = (int32_t)fp64int::hi32((uint64_t)D[i]);
+        most |= (uint32_t)(h ^ (h >> 31));
+    }
+    return most < (1u << (21 - M));
+}
+
 // Row ROW of the MRT transform applied to f: the reference sums M[ROW][i] * f[i] from 0.0 in
 // column order.  Terms with M = 0 add +-0 and are left out; products by +-1 are exact.
 template <int ROW>
@@ -205,11 +250,16 @@ __device__ __forceinline__ bool exact_sums(const double *f, const double *feq, c
     return (int)(most >> 20) + M <= (least >> 20);
 }
 
-template <int OP>
+template <int OP, bool FIXED>
 __device__ __forceinline__ void collide9(double f[9], const Relax &R)
 {
     double rho, ux, uy, feq[9];
-    moments9(f, rho, ux, uy);
+    int64_t F[9];
+    const bool fixed = FIXED && fixed_form<9>(f);
+    if (fixed)
+        moments9_fixed(f, F, rho, ux, uy);
+    else
+        moments9(f, rho, ux, uy);
     equilibrium9_int(rho, ux, uy, feq);
     if constexpr (OP == OP_MRT) {
         collide9_mrt(f, R, feq);
@@ -220,19 +270,28 @@ __device__ __forceinline__ void collide9(double f[9], const Relax &R)
         for (int i = 0; i < 9; i++) f[i] = f[i] + (feq[i] - f[i]) * R.inv_tau;
         return;
     }
-    double d[9];
+    double d[9], pxx, pyy, pxy;
+    int64_t D[9];
+    if (fixed && fixed_parts<9, 3>(F, feq, D)) {
+        const int64_t s56 = D[5] + D[6], s78 = D[7] + D[8], t = s56 + s78;
+        pxx = fp64int::to_double((D[1] + D[2]) + t);
+        pyy = fp64int::to_double((D[3] + D[4]) + t);
+        pxy = fp64int::to_double(s56 - s78);
 #pragma unroll
-    for (int i = 0; i < 9; i++) d[i] = f[i] - feq[i];
-    double pxx, pyy, pxy;
-    if (exact_sums<9, 3>(f, feq, d)) {
-        const double s56 = d[5] + d[6], s78 = d[7] + d[8], t = s56 + s78;
-        pxx = (d[1] + d[2]) + t;
-        pyy = (d[3] + d[4]) + t;
-        pxy = s56 - s78;
+        for (int i = 0; i < 9; i++) d[i] = fp64int::to_double(D[i]);
     } else {
-        pxx = ((((d[1] + d[2]) + d[5]) + d[6]) + d[7]) + d[8];
-        pyy = ((((d[3] + d[4]) + d[5]) + d[6]) + d[7]) + d[8];
-        pxy = ((d[5] + d[6]) - d[7]) - d[8];
+#pragma unroll
+        for (int i = 0; i < 9; i++) d[i] = f[i] - feq[i];
+        if (!FIXED && exact_sums<9, 3>(f, feq, d)) {
+            const double s56 = d[5] + d[6], s78 = d[7] + d[8], t = s56 + s78;
+            pxx = (d[1] + d[2]) + t;
+            pyy = (d[3] + d[4]) + t;
+            pxy = s56 - s78;
+        } else {
+            pxx = ((((d[1] + d[2]) + d[5]) + d[6]) + d[7]) + d[8];
+            pyy = ((((d[3] + d[4]) + d[5]) + d[6]) + d[7]) + d[8];
+            pxy = ((d[5] + d[6]) - d[7]) - d[8];
+        }
     }
     const double xa = QA * pxx, xb = QB * pxx, ya = QA * pyy, yb = QB * pyy;
     const double dd = xa + ya;
@@ -298,6 +357,30 @@ __device__ __forceinline__ void equilibrium19(double rho, double ux, double uy, 
     feq_pair(zmy, zmy * zmy, wr2, C, feq[17], feq[18]);
 }
 
+// moments19 in fixed point, as moments9_fixed: 45 FP64 operations less.
+__device__ __forceinline__ void moments19_fixed(const double f[19], int64_t F[19], double &rho, double &ux, double &uy,
+                                                double &uz)
+{
+    using fp64int::round53;
+#pragma unroll
+    for (int i = 0; i < 19; i++) F[i] = fp64int::to_fixed(f[i]);
+    int64_t r = F[0];
+#pragma unroll
+    for (int i = 1; i < 19; i++) r = round53(r + F[i]);
+    int64_t mx = round53(F[1] - F[2]), my = round53(F[3] - F[4]), mz = round53(F[5] - F[6]);
+#pragma unroll
+    for (int i = 7; i < 19; i++) {
+        if (Lat<19>::cx(i)) mx = round53(Lat<19>::cx(i) > 0 ? mx + F[i] : mx - F[i]);
+        if (Lat<19>::cy(i)) my = round53(Lat<19>::cy(i) > 0 ? my + F[i] : my - F[i]);
+        if (Lat<19>::cz(i)) mz = round53(Lat<19>::cz(i) > 0 ? mz + F[i] : mz - F[i]);
+    }
+    rho = fp64int::to_double(r);
+    const double inv = 1.0 / rho;
+    ux = fp64int::to_double(mx) * inv;
+    uy = fp64int::to_double(my) * inv;
+    uz = fp64int::to_double(mz) * inv;
+}
+
 __device__ __forceinline__ void equilibrium19_int(double rho, double ux, double uy, double uz, double feq[19])
 {
     const double xpy = ux + uy, xmy = ux - uy, xpz = ux + uz, xmz = ux - uz, ypz = uy + uz, zmy = uz - uy;
@@ -323,38 +406,57 @@ __device__ __forceinline__ void equilibrium19_int(double rho, double ux, double 
     feq_pair_int(zmy, zmy * zmy, wr2, C62, feq[17], feq[18]);
 }
 
-template <int OP>
+template <int OP, bool FIXED>
 __device__ __forceinline__ void collide19(double f[19], const Relax &R)
 {
     double rho, ux, uy, uz, feq[19];
-    moments19(f, rho, ux, uy, uz);
+    int64_t F[19];
+    const bool fixed = FIXED && fixed_form<19>(f);
+    if (fixed)
+        moments19_fixed(f, F, rho, ux, uy, uz);
+    else
+        moments19(f, rho, ux, uy, uz);
     equilibrium19_int(rho, ux, uy, uz, feq);
     if (OP == OP_BGK) {
 #pragma unroll
         for (int i = 0; i < 19; i++) f[i] = f[i] + (feq[i] - f[i]) * R.inv_tau;
         return;
     }
-    double d[19];
+    double d[19], pxx, pyy, pzz, pxy, pxz, pyz;
+    int64_t D[19];
+    if (fixed && fixed_parts<19, 4>(F, feq, D)) {
+        const int64_t a = D[7] + D[8], b = D[9] + D[10], ab = a + b;
+        const int64_t g = D[11] + D[12], h = D[13] + D[14], gh = g + h;
+        const int64_t m = D[15] + D[16], n = D[17] + D[18], mn = m + n;
+        pxx = fp64int::to_double((D[1] + D[2]) + (ab + gh));
+        pyy = fp64int::to_double((D[3] + D[4]) + (ab + mn));
+        pzz = fp64int::to_double((D[5] + D[6]) + (gh + mn));
+        pxy = fp64int::to_double(a - b);
+        pxz = fp64int::to_double(g - h);
+        pyz = fp64int::to_double(m - n);
 #pragma unroll
-    for (int i = 0; i < 19; i++) d[i] = f[i] - feq[i];
-    double pxx, pyy, pzz, pxy, pxz, pyz;
-    if (exact_sums<19, 4>(f, feq, d)) {
-        const double a = d[7] + d[8], b = d[9] + d[10], ab = a + b;
-        const double g = d[11] + d[12], h = d[13] + d[14], gh = g + h;
-        const double m = d[15] + d[16], n = d[17] + d[18], mn = m + n;
-        pxx = (d[1] + d[2]) + (ab + gh);
-        pyy = (d[3] + d[4]) + (ab + mn);
-        pzz = (d[5] + d[6]) + (gh + mn);
-        pxy = a - b;
-        pxz = g - h;
-        pyz = m - n;
+        for (int i = 0; i < 19; i++) d[i] = fp64int::to_double(D[i]);
     } else {
-        pxx = ((((((((d[1] + d[2]) + d[7]) + d[8]) + d[9]) + d[10]) + d[11]) + d[12]) + d[13]) + d[14];
-        pyy = ((((((((d[3] + d[4]) + d[7]) + d[8]) + d[9]) + d[10]) + d[15]) + d[16]) + d[17]) + d[18];
-        pzz = ((((((((d[5] + d[6]) + d[11]) + d[12]) + d[13]) + d[14]) + d[15]) + d[16]) + d[17]) + d[18];
-        pxy = ((d[7] + d[8]) - d[9]) - d[10];
-        pxz = ((d[11] + d[12]) - d[13]) - d[14];
-        pyz = ((d[15] + d[16]) - d[17]) - d[18];
+#pragma unroll
+        for (int i = 0; i < 19; i++) d[i] = f[i] - feq[i];
+        if (!FIXED && exact_sums<19, 4>(f, feq, d)) {
+            const double a = d[7] + d[8], b = d[9] + d[10], ab = a + b;
+            const double g = d[11] + d[12], h = d[13] + d[14], gh = g + h;
+            const double m = d[15] + d[16], n = d[17] + d[18], mn = m + n;
+            pxx = (d[1] + d[2]) + (ab + gh);
+            pyy = (d[3] + d[4]) + (ab + mn);
+            pzz = (d[5] + d[6]) + (gh + mn);
+            pxy = a - b;
+            pxz = g - h;
+            pyz = m - n;
+        } else {
+            pxx = ((((((((d[1] + d[2]) + d[7]) + d[8]) + d[9]) + d[10]) + d[11]) + d[12]) + d[13]) + d[14];
+            pyy = ((((((((d[3] + d[4]) + d[7]) + d[8]) + d[9]) + d[10]) + d[15]) + d[16]) + d[17]) + d[18];
+            pzz = ((((((((d[5] + d[6]) + d[11]) + d[12]) + d[13]) + d[14]) + d[15]) + d[16]) + d[17]) + d[18];
+            pxy = ((d[7] + d[8]) - d[9]) - d[10];
+            pxz = ((d[11] + d[12]) - d[13]) - d[14];
+            pyz = ((d[15] + d[16]) - d[17]) - d[18];
+        }
     }
     const double xa = QA * pxx, xb = QB * pxx;
     const double ya = QA * pyy, yb = QB * pyy;
@@ -386,14 +488,14 @@ __device__ __forceinline__ void collide19(double f[19], const Relax &R)
     }
 }
 
-template <int Q, int OP>
+template <int Q, int OP, bool FIXED = true>
 __device__ __forceinline__ void collide(double *f, const Relax &R)
 {
     static_assert(Q == 9 || OP != OP_MRT, "MRT is a D2Q9 operator");
     if constexpr (Q == 9)
-        collide9<OP>(f, R);
+        collide9<OP, FIXED>(f, R);
     else
-        collide19<OP>(f, R);
+        collide19<OP, FIXED>(f, R);
 }
 
 // calcula velocity of one node (for kinectic_energy, Other_functions.cpp:100-115):

@@ -106,5 +106,59 @@ __host__ __device__ __forceinline__ void eq_pair(double cv, double cv2, uint64_t
     minus = from_bits(neg ? up : uq);
 }
 
+// ---- populations in fixed point --------------------------------------------------------------------------------
+// A population 2^-6 <= f < 1 is a whole number of units of 2^-58 below 2^58.
+
+constexpr int FIX_E0 = 1017;  // exponent field of 2^-6
+
+// max over values of this is below FIX_SPAN when all of them are in range (negative ones and NaN are not)
+constexpr uint32_t FIX_SPAN = 6u << 20;
+__host__ __device__ __forceinline__ uint32_t fix_range(double f) { return hi32(bits(f)) - ((uint32_t)FIX_E0 << 20); }
+
+__host__ __device__ __forceinline__ int64_t to_fixed(double f)
+{
+    const uint64_t b = bits(f);
+    return (int64_t)(mantissa(b) << (((hi32(b) >> 20) - FIX_E0) & 7u));
+}
+
+__host__ __device__ __forceinline__ int clz32(uint32_t x)
+{
+#ifdef __CUDA_ARCH__
+    return __clz((int)x);
+#else
+    return x ? __builtin_clz(x) : 32;
+#endif
+}
+__host__ __device__ __forceinline__ int clz64(uint64_t x)
+{
+#ifdef __CUDA_ARCH__
+    return __clzll((long long)x);
+#else
+    return x ? __builtin_clzll(x) : 64;
+#endif
+}
+
+// x rounded to 53 significant bits, ties to even (|x| < 2^62).  Rounding by the floor of x + half works on
+// two's complement as it is; the magnitude's leading bit is found on x or its complement.
+__host__ __device__ __forceinline__ int64_t round53(int64_t x)
+{
+    const int32_t h = (int32_t)hi32((uint64_t)x);
+    const int k0 = 11 - clz32((uint32_t)(h ^ (h >> 31)));
+    const int k = k0 > 0 ? k0 : 0;
+    const uint32_t mask = (1u << k) - 1;
+    const uint64_t r = (uint64_t)x + (mask >> 1) + (((uint32_t)x >> k) & mask & 1u);
+    return (int64_t)(r & ~(uint64_t)mask);
+}
+
+// A fixed-point number of at most 53 significant bits as a double.
+__host__ __device__ __forceinline__ double to_double(int64_t x)
+{
+    const uint64_t a = x < 0 ? 0 - (uint64_t)x : (uint64_t)x;
+    const int lz = clz64(a) & 63;
+    const uint64_t m = (a << lz) >> 11;  // leading bit at 52: it adds 1 to the exponent field
+    const uint64_t b = m + ((uint64_t)(uint32_t)(1027 - lz) << 52);
+    return from_bits(a == 0 ? 0 : b | ((uint64_t)x & 0x8000000000000000ull));
+}
+
 }  // namespace fp64int
 }  // namespace erlbm

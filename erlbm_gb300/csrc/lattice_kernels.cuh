@@ -113,6 +113,16 @@ struct PrecExact64 {
     __device__ static __forceinline__ double to_f(T v, int) { return v; }
 };
 
+// The exact path for lattices of fewer warps than hide the latency of the fixed-point sums: the same bits with
+// more FP64 operations and fewer dependent integer ones.
+struct PrecExact64Small : PrecExact64 {
+    template <int Q, int OP>
+    __device__ static __forceinline__ void collide(T *f, const CollParams &p)
+    {
+        exact::collide<Q, OP, false>(f, p.R);
+    }
+};
+
 struct PrecShifted32 {
     using T = float;
     template <int Q, int OP>

@@ -44,6 +44,24 @@ int main(int argc, char **argv)
         cases++;
         bad += bits(p) != bits(a) || bits(m) != bits(b);
     }
+    // chains of adds and subtractions of populations in fixed point against the FP64 chain
+    for (long it = 0; it < n; it++) {
+        double s = 0;
+        int64_t S = 0;
+        for (int k = 0; k < 6; k++) {
+            double f = std::ldexp(0.5 + std::ldexp((double)(rng() >> 12), -53), -(int)(rng() % 6));
+            if (rng() % 4 == 0) f = std::ldexp(std::floor(std::ldexp(f, 20)), -20);
+            const bool in = fix_range(f) < FIX_SPAN;
+            bad += !in || to_double(to_fixed(f)) != f;
+            const bool minus = rng() % 2;
+            s = k == 0 ? f : minus ? s - f : s + f;
+            S = k == 0 ? to_fixed(f) : round53(minus ? S - to_fixed(f) : S + to_fixed(f));
+            bad += bits(to_double(S)) != bits(s + 0.0);
+            cases++;
+        }
+    }
+    const double out[] = {1.0, 1.5, 0x1p-7, 0x1.fffffffffffffp-7, -0.1, 0.0, -0.0, INFINITY, -INFINITY, NAN};
+    for (double x : out) bad += fix_range(x) < FIX_SPAN;
     printf("%ld %ld\n", cases, bad);
     return 0;
 }
