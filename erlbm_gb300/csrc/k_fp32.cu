@@ -69,6 +69,7 @@ template <int OP, int BLOCK, bool STREAMING>
 __global__ void __launch_bounds__(BLOCK) k_periodic_d2q9(const float *__restrict__ src, float *__restrict__ dst, int nx,
                                                           int ny, long long plane, shifted::Coef k)
 {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const int wpr = nx >> 7;  // warps per row
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -120,7 +121,7 @@ void go_periodic(const Geo &g, const shifted::Coef &k, const float *src, float *
 {
     const long long warps = (long long)(g.nx / 128) * g.ny;
     const unsigned nb = (unsigned)((warps * 32 + BLOCK - 1) / BLOCK);
-    k_periodic_d2q9<OP, BLOCK, ST><<<nb, BLOCK, 0, s>>>(src, dst, g.nx, g.ny, g.plane, k);
+    launch_step_kernel<k_periodic_d2q9<OP, BLOCK, ST>, BLOCK>(nb, s, src, dst, g.nx, g.ny, g.plane, k);
 }
 
 template <int OP>
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(128) k_periodic_d2q9_x2s(const float *__restri
                                                           int nx, int ny, long long plane, int hc, int strips,
                                                           int n_warps, shifted::Coef k)
 {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const int wid = (int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
     if (wid >= n_warps) return;  // the whole warp leaves together
@@ -314,6 +316,7 @@ __global__ void __launch_bounds__(128, 4) k_periodic_d2q9_x3s(const float *__res
                                                           int n_warps, const uint8_t *__restrict__ dist,
                                                           shifted::Coef k)
 {
+    after_previous();
     const int lane = threadIdx.x & 31;
     const int wid = (int)blockIdx.x * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
     if (wid >= n_warps) return;
@@ -537,6 +540,7 @@ __global__ void __launch_bounds__(128, MINB) k_periodic_d2q9_x3a(const float *__
                                                                 int n_warps, const uint8_t *__restrict__ dist,
                                                                 shifted::Coef k)
 {
+    after_previous();
     extern __shared__ __align__(16) float xa_smem[];
     const int lane = threadIdx.x & 31;
     const int wib = (int)(threadIdx.x >> 5);
@@ -682,27 +686,26 @@ bool periodic_d2q9_strips_ok(const Geo &g)
     return g.solid == nullptr && g.nz == 1 && g.nx >= 32 && g.ny >= 8;
 }
 
+// The strips' CTAs are sized for one wave.  A full wave after another comes in one for one as its CTAs leave; a part
+// of a wave, unless two fit, would crowd the SMs with room (512 x 1024 by 64-column strips 4.3 -> 5.2 us a step), and so
+// would strips after the small CTAs of the listed nodes (SKIP: 4096 x 1024 channel 28.6 -> 32.3).  Beyond some 3 million
+// nodes a launch's gap is below 2 % of it and the CTAs' drifting apart costs more (4096^2 76.5 -> 78.6).
+template <bool SKIP, class K, class... A>
+static void launch_strips(K kern, int n_warps, int resident, size_t smem, cudaStream_t s, const float *src, float *dst,
+                          int nx, int ny, A... args)
+{
+    const bool early = !SKIP && (2LL * n_warps <= resident || 10LL * n_warps >= 9LL * resident) &&
+                       (long long)nx * ny < 3000000;
+    launch_after(early, kern, (unsigned)((n_warps + 3) / 4), 128, smem, s, src, dst, nx, ny, args...);
+}
+
 // Two-step launch: 128-thread CTAs of four independent warps, and rows per chunk such that one wave
 // of resident warps covers the ceil(nx / 30) x (ny / hc) warp strips (no second, partial wave).
 template <int OP>
 static void go_x2(const Geo &g, const shifted::Coef &k, const float *src, float *dst, cudaStream_t s)
 {
-    auto kern = k_periodic_d2q9_x2s<OP>;
-    // resident warps per device, found once per device and instantiation (handles on several host
-    // threads may launch concurrently; they store the same value)
-    constexpr int MAXDEV = 64;
-    static std::atomic<int> warps_cache[MAXDEV];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int d = dev >= 0 && dev < MAXDEV ? dev : 0;
-    int resident = warps_cache[d].load(std::memory_order_relaxed);
-    if (resident <= 0) {
-        int o = 0, n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, 128, 0) != cudaSuccess || o < 1) o = 1;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        resident = o * 4 * (n > 0 ? n : 1);
-        warps_cache[d].store(resident, std::memory_order_relaxed);
-    }
+    constexpr auto KERN = k_periodic_d2q9_x2s<OP>;
+    const int resident = 4 * resident_ctas<KERN, 128>();  // warps
     const int strips = (g.nx + XS_W - 1) / XS_W;
     const long long slots = resident;
     long long chunks = slots / strips;
@@ -712,8 +715,7 @@ static void go_x2(const Geo &g, const shifted::Coef &k, const float *src, float 
     hc += hc & 1;
     if (hc > g.ny) hc = g.ny;
     const int n_warps = strips * (int)((g.ny + hc - 1) / hc);
-    const unsigned nb = (unsigned)((n_warps + 3) / 4);
-    kern<<<nb, 128, 0, s>>>(src, dst, g.nx, g.ny, g.plane, (int)hc, strips, n_warps, k);
+    launch_strips<false>(KERN, n_warps, resident, 0, s, src, dst, g.nx, g.ny, g.plane, (int)hc, strips, n_warps, k);
 }
 
 // Three-step launch: as go_x2, over ceil(nx / 28) strips.
@@ -721,20 +723,8 @@ template <int OP, bool SKIP = false>
 static void go_x3(const Geo &g, const shifted::Coef &k, const float *src, float *dst, cudaStream_t s,
                   const uint8_t *dist = nullptr)
 {
-    auto kern = k_periodic_d2q9_x3s<OP, SKIP>;
-    constexpr int MAXDEV = 64;
-    static std::atomic<int> warps_cache[MAXDEV];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int d = dev >= 0 && dev < MAXDEV ? dev : 0;
-    int resident = warps_cache[d].load(std::memory_order_relaxed);
-    if (resident <= 0) {
-        int o = 0, n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, 128, 0) != cudaSuccess || o < 1) o = 1;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        resident = o * 4 * (n > 0 ? n : 1);
-        warps_cache[d].store(resident, std::memory_order_relaxed);
-    }
+    constexpr auto KERN = k_periodic_d2q9_x3s<OP, SKIP>;
+    const int resident = 4 * resident_ctas<KERN, 128>();  // warps
     const int strips = (g.nx + X3_W - 1) / X3_W;
     const long long slots = resident;
     long long chunks = slots / strips;
@@ -744,7 +734,7 @@ static void go_x3(const Geo &g, const shifted::Coef &k, const float *src, float 
     hc += hc & 1;
     if (hc > g.ny) hc = g.ny;
     const int n_warps = strips * (int)((g.ny + hc - 1) / hc);
-    kern<<<(unsigned)((n_warps + 3) / 4), 128, 0, s>>>(src, dst, g.nx, g.ny, g.plane, (int)hc, strips, n_warps, dist, k);
+    launch_strips<SKIP>(KERN, n_warps, resident, 0, s, src, dst, g.nx, g.ny, g.plane, (int)hc, strips, n_warps, dist, k);
 }
 
 // Three-step launch over column pairs: ceil(nx / 60) strips, chunks of whole unrolled groups, as many
@@ -755,21 +745,9 @@ template <int OP, bool SKIP = false>
 static void go_x3a(const Geo &g, const shifted::Coef &k, const float *src, float *dst, cudaStream_t s,
                    const uint8_t *dist = nullptr)
 {
-    auto kern = k_periodic_d2q9_x3a<OP, XA_MINB, SKIP>;
+    constexpr auto KERN = k_periodic_d2q9_x3a<OP, XA_MINB, SKIP>;
     const size_t smem = 4 * XA_SMEM_PER_WARP;
-    constexpr int MAXDEV = 64;
-    static std::atomic<int> warps_cache[MAXDEV];
-    int dev = 0;
-    cudaGetDevice(&dev);
-    const int d = dev >= 0 && dev < MAXDEV ? dev : 0;
-    int resident = warps_cache[d].load(std::memory_order_relaxed);
-    if (resident <= 0) {
-        int o = 0, n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&o, kern, 128, smem) != cudaSuccess || o < 1) o = 1;
-        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-        resident = o * 4 * (n > 0 ? n : 1);
-        warps_cache[d].store(resident, std::memory_order_relaxed);
-    }
+    const int resident = 4 * resident_ctas<KERN, 128>(smem);  // warps
     const int strips = (g.nx + XP_W - 1) / XP_W;
     long long chunks = resident / strips;
     if (chunks < 1) chunks = 1;
@@ -777,7 +755,7 @@ static void go_x3a(const Geo &g, const shifted::Coef &k, const float *src, float
     hc = (hc + XP_SPAN - 1) / XP_SPAN * XP_SPAN;
     if (hc < 2 * XP_SPAN) hc = 2 * XP_SPAN;
     const int n_warps = strips * (int)((g.ny + hc - 1) / hc);
-    kern<<<(unsigned)((n_warps + 3) / 4), 128, smem, s>>>(src, dst, g.nx, g.ny, (int)g.plane, (int)hc, strips, n_warps,
+    launch_strips<SKIP>(KERN, n_warps, resident, smem, s, src, dst, g.nx, g.ny, (int)g.plane, (int)hc, strips, n_warps,
                                                          dist, k);
 }
 
@@ -920,6 +898,7 @@ __global__ void __launch_bounds__(128, 6) k_periodic_d3q19(const float *__restri
                                                             unsigned nx, unsigned ny, unsigned nz, unsigned nbox,
                                                             size_t plane, FastDiv fx, FastDiv fy, shifted::Coef k)
 {
+    after_previous();
     const unsigned node = blockIdx.x * 128u + threadIdx.x;
     if (node >= nbox) return;
     const unsigned r = fdiv(node, fx), x = node - r * nx, z = fdiv(r, fy), y = r - z * ny;
@@ -954,9 +933,9 @@ int launch_periodic_d3q19_fp32(int op, const Geo &g, const Relax &R, const float
     const unsigned nx = (unsigned)g.nx, ny = (unsigned)g.ny, nz = (unsigned)g.nz;
     const size_t pl = (size_t)g.plane;
     switch (op) {
-    case OP_BGK: k_periodic_d3q19<OP_BGK><<<nb, 128, 0, s>>>(src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
-    case OP_REG: k_periodic_d3q19<OP_REG><<<nb, 128, 0, s>>>(src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
-    case OP_EXTREG: k_periodic_d3q19<OP_EXTREG><<<nb, 128, 0, s>>>(src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
+    case OP_BGK: launch_step_kernel<k_periodic_d3q19<OP_BGK>, 128>(nb, s, src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
+    case OP_REG: launch_step_kernel<k_periodic_d3q19<OP_REG>, 128>(nb, s, src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
+    case OP_EXTREG: launch_step_kernel<k_periodic_d3q19<OP_EXTREG>, 128>(nb, s, src, dst, nx, ny, nz, n, pl, fx, fy, k); break;
     default: return -1;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
@@ -989,6 +968,7 @@ __global__ void __launch_bounds__(256) k_d2q9_hybrid(const float *__restrict__ s
                                                      const uint8_t *__restrict__ nodeflag,
                                                      const int *__restrict__ fix, int n_fix, int n_fix_blocks)
 {
+    after_previous();
     const int nx = g.nx, ny = g.ny;
     const long long plane = g.plane;
     if ((int)blockIdx.x < n_fix_blocks) {
@@ -1134,11 +1114,11 @@ int launch_step_fp32_hybrid(int op, const Geo &g, const BCp &bc, const Relax &R,
     if (nb > 0x7fffffffLL) return -1;
     const int fb = (int)fix_blocks;
     switch (op) {
-    case OP_BGK: k_d2q9_hybrid<OP_BGK><<<(unsigned)nb, 256, 0, s>>>(src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb); break;
-    case OP_MRT: k_d2q9_hybrid<OP_MRT><<<(unsigned)nb, 256, 0, s>>>(src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb); break;
-    case OP_REG: k_d2q9_hybrid<OP_REG><<<(unsigned)nb, 256, 0, s>>>(src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb); break;
+    case OP_BGK: launch_step_kernel<k_d2q9_hybrid<OP_BGK>, 256>((unsigned)nb, s, src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb); break;
+    case OP_MRT: launch_step_kernel<k_d2q9_hybrid<OP_MRT>, 256>((unsigned)nb, s, src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb); break;
+    case OP_REG: launch_step_kernel<k_d2q9_hybrid<OP_REG>, 256>((unsigned)nb, s, src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb); break;
     case OP_EXTREG:
-        k_d2q9_hybrid<OP_EXTREG><<<(unsigned)nb, 256, 0, s>>>(src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb);
+        launch_step_kernel<k_d2q9_hybrid<OP_EXTREG>, 256>((unsigned)nb, s, src, dst, g, bc, prm, segflag, nodeflag, fix, n_fix, fb);
         break;
     default: return -1;
     }
@@ -1210,12 +1190,13 @@ __global__ void __launch_bounds__(256) k_fix_list(Geo g, const uint8_t *__restri
 // One generic step at the nodes of the planes and the first n_list listed ones.  Bound by latency (list entry,
 // populations, collision, and on a plane its FP64 closure: about 75 cycles per dependent FP64 operation), so
 // the plane nodes have warps of their own: among the others, in row order, one of them would hold up a
-// warp per row (9.2 -> @LS@ us per launch on the 4096 x 1024 channel).
+// warp per row (9.2 -> 6.8 us per launch on the 4096 x 1024 channel).
 template <int OP>
 __global__ void __launch_bounds__(64) k_listed_step(const float *__restrict__ src, float *__restrict__ dst, Geo g,
                                                     BCp bc, shifted::Coef k, const int *__restrict__ list, int n_list,
                                                     int n_planes)
 {
+    after_previous();
     int t = (int)(blockIdx.x * 64 + threadIdx.x);
     int x, y, node;
     float f[9];
@@ -1255,8 +1236,8 @@ void go_planes_x3(const Geo &g, const BCp &bc, const shifted::Coef &k, const flo
     const int planes = ((bc.inlet_x >= 0 ? g.ny : 0) + (bc.outlet_x >= 0 ? g.ny : 0) + (bc.open_y >= 0 ? g.nx : 0) + 31) / 32 * 32;
     auto listed = [&](const float *from, float *to, int count) {
         if (planes + count > 0)
-            k_listed_step<OP><<<(unsigned)((planes + count + 63) / 64), 64, 0, s>>>(from, to, g, bc, k, list, count,
-                                                                                   planes);
+            launch_after(true, k_listed_step<OP>, (unsigned)((planes + count + 63) / 64), 64, 0, s, from, to, g, bc, k, list,
+                         count, planes);
     };
     listed(src, dst, n[0] + n[1] + n[2]);
     listed(dst, mid, n[0] + n[1]);
@@ -1272,7 +1253,9 @@ void go_planes_x3(const Geo &g, const BCp &bc, const shifted::Coef &k, const flo
 // From the sizes on where three steps by threes beat three single steps: a launch sequence costs three
 // latency-bound listed launches (about 5 us each), whatever the size, and saves two thirds of the traffic, or, where
 // nx % 128 != 0, the generic per-node kernel.  Measured on channels, us per step, single against threes:
-// @RULE@
+// fused single steps (nx % 128 == 0) 4096 x 1024 46.9 / 28.6, 2048 x 512 10.7 / 12.1, 1536 x 384 10.5 / 10.3, 512 x 128
+// 7.8 / 7.3; generic single steps 3000 x 1500 98.9 / 29.6, 2800 x 700 47.0 / 17.5, 1000 x 250 10.3 / 7.7, 500 x 125
+// 4.5 / 7.7.
 bool d2q9_planes_x3_ok(const Geo &g)
 {
     return g.nz == 1 && g.nx >= 32 && g.ny >= 16 && g.nbox < (1LL << 31) - 256 &&
@@ -1304,7 +1287,8 @@ int d2q9_fix_list(const Geo &g, const uint8_t *fix, const uint8_t *dist, int *at
 // populations that are not theirs; nothing they store depends on those.  Every stored value is the generic
 // kernel's, bit for bit.
 // HBM bytes per update drop from 72 to 24 plus the listed nodes': 4096 x 1024 with walls, a cylinder and two
-// planes (@LIST@ listed nodes): @CH0@ us per three steps in single steps -> @CH1@ us.
+// planes, 141 us per three single steps -> 86 us, of which the strips take 65 (bound as k_periodic_d2q9_x3a) and
+// the three listed launches some 7 each.
 int launch_d2q9_planes_x3(int op, const Geo &g, const BCp &bc, const Relax &R, const float *src, float *dst, float *mid,
                           const uint8_t *dist, const int *list, const int n[3], cudaStream_t s)
 {

@@ -19,6 +19,7 @@
 #include "collide_fp64.cuh"
 #include "kernels_api.h"
 #include "lattice.cuh"
+#include "launch.cuh"
 
 namespace erlbm {
 
@@ -425,6 +426,7 @@ template <class P, int Q, int OP>
 __global__ void __launch_bounds__(256) k_step(const typename P::T *__restrict__ src, typename P::T *__restrict__ dst,
                                               Geo g, BCp bc, CollParams prm, StepArgs a)
 {
+    after_previous();
     if (a.stop_on_flag && a.status != nullptr) {
         // A check failed in an EARLIER step: nothing to do.  (Blocks of the failing step itself
         // still finish it, as the reference finishes the step in which it flags a node.)  One
@@ -594,20 +596,20 @@ int step_dispatch(int op, const Geo &g, const BCp &bc, const Relax &R, const Ste
     const unsigned nb = blocks_for(g.nbox, bs);
     switch (op) {
     case OP_BGK:
-        k_step<P, Q, OP_BGK><<<nb, bs, 0, s>>>(src, dst, g, bc, prm, a);
+        launch_step_kernel<k_step<P, Q, OP_BGK>, bs>(nb, s, src, dst, g, bc, prm, a);
         break;
     case OP_MRT:
         if constexpr (Q == 9) {
-            k_step<P, Q, OP_MRT><<<nb, bs, 0, s>>>(src, dst, g, bc, prm, a);
+            launch_step_kernel<k_step<P, Q, OP_MRT>, bs>(nb, s, src, dst, g, bc, prm, a);
             break;
         } else {
             return -1;
         }
     case OP_REG:
-        k_step<P, Q, OP_REG><<<nb, bs, 0, s>>>(src, dst, g, bc, prm, a);
+        launch_step_kernel<k_step<P, Q, OP_REG>, bs>(nb, s, src, dst, g, bc, prm, a);
         break;
     case OP_EXTREG:
-        k_step<P, Q, OP_EXTREG><<<nb, bs, 0, s>>>(src, dst, g, bc, prm, a);
+        launch_step_kernel<k_step<P, Q, OP_EXTREG>, bs>(nb, s, src, dst, g, bc, prm, a);
         break;
     default:
         return -1;

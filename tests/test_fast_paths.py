@@ -119,8 +119,8 @@ def test_three_steps_per_launch_with_planes_equal_single_steps(nx, ny, op, plane
         f = (w[None, :] * (1.0 + 0.03 * rng.standard_normal((a.n_fluid, 9)))).ravel()
         a.set_populations(f)
         b.set_populations(f)
-        a.step(72, bc)
-        for _ in range(72):
+        a.step(200, bc)
+        for _ in range(200):
             b.step(1, bc)
         assert np.array_equal(a.get_populations(E.STAGE_POST_COLLISION), b.get_populations(E.STAGE_POST_COLLISION))
         assert np.array_equal(a.get_populations(), b.get_populations())
