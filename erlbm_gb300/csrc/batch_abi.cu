@@ -61,12 +61,23 @@ struct Scratch {
 
 namespace erlbm {
 
-int pick_shape(int prec, int q, int nb, int slots, int n_runs, LaunchShape *out)
+int launch_batch(int prec, int q, const BatchGeo &g, const BatchRun *runs, int n_runs, int *counter, BatchResult *res,
+                 const double *aos, const LaunchShape &sh, cudaStream_t s)
 {
+    if (sh.mirror) return launch_batch_mirror(g, runs, n_runs, counter, res, sh, s);
+    const auto launch = prec == ERLBM_FP64 ? launch_batch_fp64 : launch_batch_fp32;
+    return launch(q, sh.npt, g, runs, n_runs, counter, res, aos, sh.grid, sh.block, sh.smem, sh.dbl, s);
+}
+
+int pick_shape(int prec, int q, const BatchGeo &g, int slots, int n_runs, LaunchShape *out)
+{
+    const int nb = g.nb;
+    out->mirror = batch_mirror_ok(prec, q, g) && batch_mirror_shape(g, slots, sm_count(), n_runs, out) == 0;
+    if (out->mirror) return ERLBM_OK;
     static const int NPT_64[] = {1, 2, 4};
     // FP32 prefers two nodes per thread (more independent work per thread; D2Q9 pairs also collide in
-    // packed FP32x2 instructions): Taylor-Green map on GB300 42.2 k runs/s against 33.9 k with one
-    // node per thread
+    // packed FP32x2 instructions): Taylor-Green map (k_batch) on GB300 42.2 k runs/s against 33.9 k with
+    // one node per thread
     static const int NPT_32[] = {2, 1, 4, 8};
     const int *list = prec == ERLBM_FP64 ? NPT_64 : NPT_32;
     const int nl = prec == ERLBM_FP64 ? 3 : 4;
@@ -158,9 +169,6 @@ int run_batch(const erlbm_batch_desc *d, int n_runs, const erlbm_run_spec *runs,
         r.op = s.op;
         r.out = order[k];
     }
-    LaunchShape sh;
-    if ((rc = pick_shape(d->precision, d->q, nb, d->slots, n_runs, &sh))) return rc;
-
     Scratch m;
     BatchRun *d_runs;
     BatchResult *d_res;
@@ -209,16 +217,14 @@ int run_batch(const erlbm_batch_desc *d, int n_runs, const erlbm_run_spec *runs,
         CK(m.alloc(&d_aos, n_aos * sizeof(double)));
         CK(cudaMemcpyAsync(d_aos, aos, n_aos * sizeof(double), cudaMemcpyHostToDevice, stream));
     }
+    LaunchShape sh;
+    if ((rc = pick_shape(d->precision, d->q, g, d->slots, n_runs, &sh))) return rc;
     // counter reset + persistent kernel, captured into a CUDA graph and launched as one unit
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(d_counter, 0, sizeof(int), stream);
-    const int lrc = d->precision == ERLBM_FP64
-                        ? launch_batch_fp64(d->q, sh.npt, g, d_runs, n_runs, d_counter, d_res, d_aos, sh.grid,
-                                            sh.block, sh.smem, sh.dbl, stream)
-                        : launch_batch_fp32(d->q, sh.npt, g, d_runs, n_runs, d_counter, d_res, d_aos, sh.grid,
-                                            sh.block, sh.smem, sh.dbl, stream);
+    const int lrc = launch_batch(d->precision, d->q, g, d_runs, n_runs, d_counter, d_res, d_aos, sh, stream);
     cudaError_t ce = cudaStreamEndCapture(stream, &graph);
     if (lrc != 0 || ce != cudaSuccess) {
         if (graph) cudaGraphDestroy(graph);

@@ -159,8 +159,17 @@ int launch_batch_fp32(int q, int npt, const BatchGeo &g, const BatchRun *runs, i
 struct LaunchShape {
     int npt, block, grid, dbl;
     size_t smem;
+    bool mirror;  // k_batch_mirror instead of k_batch
 };
-int pick_shape(int prec, int q, int nb, int slots, int n_runs, LaunchShape *out);
+int pick_shape(int prec, int q, const BatchGeo &g, int slots, int n_runs, LaunchShape *out);
+// FP32 Taylor-Green map runs in mirror-symmetric form (k_map32.cu): which runs, the launch shape, the launch.
+bool batch_mirror_ok(int prec, int q, const BatchGeo &g);
+int batch_mirror_shape(const BatchGeo &g, int slots, int sms, int n_runs, LaunchShape *out);
+int launch_batch_mirror(const BatchGeo &g, const BatchRun *runs, int n_runs, int *counter, BatchResult *res,
+                        const LaunchShape &sh, cudaStream_t s);
+// The launch of pick_shape's shape.
+int launch_batch(int prec, int q, const BatchGeo &g, const BatchRun *runs, int n_runs, int *counter, BatchResult *res,
+                 const double *aos, const LaunchShape &sh, cudaStream_t s);
 
 // Resident CTAs per SM for a configuration (0 if it cannot run).
 int batch_occupancy(int prec, int q, int npt, int block, size_t smem);

@@ -211,12 +211,8 @@ extern "C" int erlbm_batch_run_noalloc(const erlbm_batch_desc *d, int n_runs, co
     k_prepare_runs<<<(n_runs + 255) / 256, 256, 0, s>>>(runs, n_runs, d->q, prepared, refused);
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "noalloc prepare");
     LaunchShape sh;
-    if ((rc = pick_shape(d->precision, d->q, g.nb, d->slots, n_runs, &sh))) return rc;
-    const int lrc = d->precision == ERLBM_FP64
-                        ? launch_batch_fp64(d->q, sh.npt, g, prepared, n_runs, counter, (BatchResult *)out, nullptr,
-                                            sh.grid, sh.block, sh.smem, sh.dbl, s)
-                        : launch_batch_fp32(d->q, sh.npt, g, prepared, n_runs, counter, (BatchResult *)out, nullptr,
-                                            sh.grid, sh.block, sh.smem, sh.dbl, s);
+    if ((rc = pick_shape(d->precision, d->q, g, d->slots, n_runs, &sh))) return rc;
+    const int lrc = launch_batch(d->precision, d->q, g, prepared, n_runs, counter, (BatchResult *)out, nullptr, sh, s);
     if (lrc == -1) {
         set_error("no batched kernel for this lattice shape%s%s", "", "");
         return ERLBM_E_UNSUPPORTED;
