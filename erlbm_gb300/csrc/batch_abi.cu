@@ -84,7 +84,10 @@ int pick_shape(int prec, int q, const BatchGeo &g, int slots, int n_runs, Launch
     for (int k = 0; k < nl; k++) {
         const int npt = list[k];
         if (q == 19 && npt > (prec == ERLBM_FP64 ? 2 : 4)) continue;
-        int block = ((nb + npt - 1) / npt + 31) / 32 * 32;
+        // a thread for every fluid node (FP64); FP32 keeps a thread for every node of the box, whose warps its
+        // energy sum follows
+        const int nodes = prec == ERLBM_FP64 ? g.n_fluid : nb;
+        int block = ((nodes + npt - 1) / npt + 31) / 32 * 32;
         if (block < 32) block = 32;
         if (block > (npt == 1 ? 288 : 512)) continue;
         // two population buffers (one barrier per step) when they fit, else one
@@ -184,6 +187,7 @@ int run_batch(const erlbm_batch_desc *d, int n_runs, const erlbm_run_spec *runs,
     g.nx = d->nx;
     g.ny = d->ny;
     g.nb = nb;
+    g.n_fluid = (int)n_fluid;
     g.inlet_x = d->inlet_x;
     g.outlet_x = d->outlet_x;
     g.rho0 = d->rho0;

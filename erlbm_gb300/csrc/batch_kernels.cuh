@@ -34,6 +34,7 @@ enum BatchInit : int { INIT_REST = 0, INIT_TG_MAP = 1, INIT_AOS = 2 };
 // Geometry and checks shared by every run of a launch.
 struct BatchGeo {
     int nx, ny, nb;               // box (nz = 1), nb = nx * ny
+    int n_fluid;                  // fluid nodes where the host knows the mask, else nb
     const uint8_t *solid;         // nb bytes, 1 = solid; null = fully periodic
     int inlet_x, outlet_x;        // boundary planes, -1 = none (D3Q19 inlet only)
     double rho0;                  // outlet density and rest density
@@ -82,23 +83,17 @@ struct BatchResult {
 };
 
 template <class P, int Q>
-__device__ __forceinline__ void batch_collide(typename P::T *f, const BatchRun &r)
+__device__ __forceinline__ uint32_t batch_collide(typename P::T *f, const BatchRun &r)  // returns the density hint
 {
     CollParams prm;
     prm.R = r.R;
     prm.k = r.k;
     if constexpr (Q == 9) {
-        if (r.op == OP_MRT) {
-            P::template collide<Q, OP_MRT>(f, prm);
-            return;
-        }
+        if (r.op == OP_MRT) return P::template collide_hint<Q, OP_MRT>(f, prm);
     }
-    if (r.op == OP_BGK)
-        P::template collide<Q, OP_BGK>(f, prm);
-    else if (r.op == OP_REG)
-        P::template collide<Q, OP_REG>(f, prm);
-    else
-        P::template collide<Q, OP_EXTREG>(f, prm);
+    if (r.op == OP_BGK) return P::template collide_hint<Q, OP_BGK>(f, prm);
+    if (r.op == OP_REG) return P::template collide_hint<Q, OP_REG>(f, prm);
+    return P::template collide_hint<Q, OP_EXTREG>(f, prm);
 }
 
 // Two D2Q9 nodes of the FP32 path at once, in the halves of float2 lanes (packed FP32x2
@@ -236,6 +231,7 @@ struct BatchSmem {
     uint8_t *solid;
     short *order;   // node of each thread slot: fluid nodes only, boundary-plane nodes first
     int *n_fluid;
+    uint32_t *known;  // upper word of the greatest density the check has seen in this run (FP64)
     double *zh;     // the run's Zou-He closure constants (P::ZouHe, <= 32 bytes)
     __device__ BatchSmem(unsigned char *raw, int nb, int dbl)
     {
@@ -246,25 +242,54 @@ struct BatchSmem {
         solid = reinterpret_cast<uint8_t *>(red + blockDim.x + 1);
         order = reinterpret_cast<short *>(solid + ((size_t)nb + 15) / 16 * 16);
         n_fluid = reinterpret_cast<int *>(order + ((size_t)nb * sizeof(short) + 15) / 16 * 16 / sizeof(short));
+        known = reinterpret_cast<uint32_t *>(n_fluid + 1);
         zh = reinterpret_cast<double *>(n_fluid + 4);
     }
 };
 
 // Thread slots of a geometry (one thread, after sm.solid is loaded): the fluid nodes in node order,
-// except that the nodes of the boundary planes come first.  Those run the inlet and outlet closures
-// (with FP64 operations in the FP32 path); packed into the first warp, they no longer put that work
-// on every warp of the CTA in every step.  Solid nodes get no thread.
-__device__ inline void make_order(const BatchGeo &g, short *order, int *n_fluid, const uint8_t *solid)
+// except that the nodes of the boundary planes are packed together.  Those run the inlet and outlet closures
+// (with FP64 operations in the FP32 path); packed, they do not put that work on every warp of the CTA in every
+// step.  Solid nodes get no thread.
+// FP32: both planes first, in one warp.  FP64 (apart): a warp's FP64 instructions hold its scheduler's pipe however
+// few of its lanes take part, so each plane gets a warp of its own, and the CTAs of the grid's second half, which
+// share their SMs with those of the first, the next two, so that four schedulers take the four planes' closures.
+__device__ inline void make_order(const BatchGeo &g, short *order, int *n_fluid, const uint8_t *solid, bool apart)
 {
-    int k = 0;
-    for (int pass = 0; pass < 2; pass++)
-        for (int n = 0; n < g.nb; n++) {
-            if (solid[n]) continue;
-            const int x = n % g.nx;
-            const bool plane = x == g.inlet_x || x == g.outlet_x;
-            if (plane == (pass == 0)) order[k++] = (short)n;
+    int n_all = 0, n_in = 0, n_out = 0;
+    for (int n = 0; n < g.nb; n++) {
+        if (solid[n]) continue;
+        const int x = n % g.nx;
+        n_all++;
+        n_in += x == g.inlet_x;
+        n_out += x == g.outlet_x && x != g.inlet_x;
+    }
+    int in = 0, out = n_in;  // first slots of the planes
+    if (apart && n_in <= 32 && n_out <= 32 && n_all >= 128) {
+        in = 2 * blockIdx.x >= gridDim.x ? 64 : 0;
+        out = in + 32;
+        if (out + n_out > n_all) {
+            in = 0;
+            out = 32;
         }
-    *n_fluid = k;
+    }
+    const int in_end = in + n_in, out_end = out + n_out;
+    int k = 0, a = in, b = out;
+    for (int n = 0; n < g.nb; n++) {
+        if (solid[n]) continue;
+        const int x = n % g.nx;
+        if (!apart && (x == g.inlet_x || x == g.outlet_x)) {
+            order[a++] = (short)n;  // node order over both planes
+        } else if (x == g.inlet_x) {
+            order[a++] = (short)n;
+        } else if (x == g.outlet_x) {
+            order[b++] = (short)n;
+        } else {
+            while ((k >= in && k < in_end) || (k >= out && k < out_end)) k++;
+            order[k++] = (short)n;
+        }
+    }
+    *n_fluid = n_all;
 }
 
 // One run of one lattice by the whole CTA.  sm.solid must hold the geometry's mask.  The result is
@@ -307,7 +332,24 @@ __device__ BatchResult batch_one_run(const BatchGeo &g, const BatchRun &r, const
     // them in registers for the whole run would cost every thread
     using ZH = typename P::ZouHe;
     static_assert(sizeof(ZH) <= 32, "ZouHe constants exceed their shared-memory slot");
-    if (tid == 0) *reinterpret_cast<ZH *>(sm.zh) = P::zou_he_prep(r.u0);
+    if (tid == 0) *reinterpret_cast<ZH *>(sm.zh) = P::zou_he_prep_run(r.u0);
+    if (tid == 0) *sm.known = 0;
+
+    // directions that come back from a solid neighbour, a bit each: found once a run, where a lookup in every step
+    // was a byte from shared memory per direction
+    uint32_t bounce[NPT];
+#pragma unroll
+    for (int s = 0; s < NPT; s++) {
+        bounce[s] = 0;
+        if (!any_solid || !fluid[s]) continue;
+        int x = nx_[s];
+        if (x == g.outlet_x) x += (g.outlet_x < g.nx / 2) ? 1 : -1;  // the outlet copies its inner neighbour
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            const int xs = wrap1(x - Lat<Q>::cx(i), g.nx), ys = wrap1(ny_[s] - Lat<Q>::cy(i), g.ny);
+            if (solid[xs + g.nx * ys]) bounce[s] |= 1u << i;
+        }
+    }
 
     // ---- initial populations (post-stream state of step 0) ----
     T f[NPT][Q];
@@ -365,7 +407,7 @@ __device__ BatchResult batch_one_run(const BatchGeo &g, const BatchRun &r, const
                     const int xs = wrap1(x - Lat<Q>::cx(i), g.nx);
                     const int ys = wrap1(y - Lat<Q>::cy(i), g.ny);
                     const int src = xs + g.nx * ys;
-                    f[s][i] = (any_solid && solid[src]) ? cur[Lat<Q>::opp(i) * NB + me] : cur[i * NB + src];
+                    f[s][i] = cur[bounce[s] >> i & 1u ? Lat<Q>::opp(i) * NB + me : i * NB + src];
                 }
             }
         } else if (g.outlet_x >= 0) {
@@ -436,7 +478,8 @@ __device__ BatchResult batch_one_run(const BatchGeo &g, const BatchRun &r, const
 #pragma unroll
         for (int s = 0; s < NPT; s++) {
             if (!fluid[s]) continue;
-            if constexpr (!PAIRS) batch_collide<P, Q>(f[s], r);
+            uint32_t hint = exact::NO_HINT;
+            if constexpr (!PAIRS) hint = batch_collide<P, Q>(f[s], r);
             if (g.density_check) {
                 if constexpr (sizeof(T) == 4) {
                     const float d = shifted::node_drho<Q>(f[s]);
@@ -447,13 +490,16 @@ __device__ BatchResult batch_one_run(const BatchGeo &g, const BatchRun &r, const
                         dmin = fminf(dmin, d);
                         if (d > g.drho_hi || d < g.drho_lo) flag |= 1;
                     }
-                } else {
+                } else if (!exact::density_below(hint, *(volatile uint32_t *)sm.known)) {
                     const double rho = P::template density<Q>(f[s]);
                     if (!isfinite(rho)) {
                         flag |= 2;
                     } else {
                         const double a = fabs(rho);
-                        max_rho = fmax(max_rho, a);
+                        if (a > max_rho) {
+                            max_rho = a;
+                            atomicMax(sm.known, (uint32_t)__double2hiint(a));
+                        }
                         if (a > g.density_limit) flag |= 1;
                     }
                 }
@@ -509,7 +555,7 @@ __global__ void __launch_bounds__(MAXT, BatchBounds<NPT, sizeof(typename P::T)>:
     const int tid = threadIdx.x;
     for (int k = tid; k < g.nb; k += blockDim.x) sm.solid[k] = g.solid ? g.solid[k] : 0;
     __syncthreads();
-    if (tid == 0) make_order(g, sm.order, sm.n_fluid, sm.solid);
+    if (tid == 0) make_order(g, sm.order, sm.n_fluid, sm.solid, sizeof(typename P::T) == 8 && NPT == 1);
     for (;;) {
         __syncthreads();
         if (tid == 0) s_run = atomicAdd(counter, 1);
@@ -614,7 +660,8 @@ __global__ void __launch_bounds__(BatchBounds<NPT, sizeof(typename P::T)>::MAXT,
         // the launch's shared memory is sized for max_nb nodes; a smaller lattice uses its prefix
         for (int k = tid; k < g.nb && k < max_nb; k += blockDim.x) sm.solid[k] = g.solid ? g.solid[k] : 0;
         __syncthreads();
-        if (tid == 0 && g.nb <= max_nb) make_order(g, sm.order, sm.n_fluid, sm.solid);
+        if (tid == 0 && g.nb <= max_nb)
+            make_order(g, sm.order, sm.n_fluid, sm.solid, sizeof(typename P::T) == 8 && NPT == 1);
         __syncthreads();
         BatchResult o;
         if (g.nb > max_nb || g.nb > NPT * (int)blockDim.x) {

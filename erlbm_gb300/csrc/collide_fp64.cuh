@@ -250,8 +250,22 @@ __device__ __forceinline__ bool exact_sums(const double *f, const double *feq, c
     return (int)(most >> 20) + M <= (least >> 20);
 }
 
+// The collision keeps a node's density up to its rounding.  Where the populations, equilibria and non-equilibrium
+// parts are in the ranges of fixed_parts or exact_sums, every rounding is below 2^-52 of the density times a
+// relaxation coefficient, so the density after the collision differs from the one before by less than 2^-21 of it
+// for coefficients below 2^10: two units of its upper word.  A density check that has seen a greater density needs no
+// sum of such a node (18 FP64 operations).  The hint is the upper word of the density, or NO_HINT.
+constexpr uint32_t NO_HINT = 0xffffffffu;
+__device__ __forceinline__ uint32_t density_hint(double rho, const Relax &R)
+{
+    const uint32_t h = (uint32_t)__double2hiint(rho);
+    return max(abs_hi(R.omega_1), abs_hi(R.omega_gt1)) < 0x40900000u ? h : NO_HINT;
+}
+// Whether a node's density after the collision is less than a density with the upper word `known`.
+__device__ __forceinline__ bool density_below(uint32_t hint, uint32_t known) { return known > 2 && hint < known - 2; }
+
 template <int OP, bool FIXED>
-__device__ __forceinline__ void collide9(double f[9], const Relax &R)
+__device__ __forceinline__ void collide9(double f[9], const Relax &R, uint32_t &hint)
 {
     double rho, ux, uy, feq[9];
     int64_t F[9];
@@ -273,6 +287,7 @@ __device__ __forceinline__ void collide9(double f[9], const Relax &R)
     double d[9], pxx, pyy, pxy;
     int64_t D[9];
     if (fixed && fixed_parts<9, 3>(F, feq, D)) {
+        hint = density_hint(rho, R);
         const int64_t s56 = D[5] + D[6], s78 = D[7] + D[8], t = s56 + s78;
         pxx = fp64int::to_double((D[1] + D[2]) + t);
         pyy = fp64int::to_double((D[3] + D[4]) + t);
@@ -283,6 +298,7 @@ __device__ __forceinline__ void collide9(double f[9], const Relax &R)
 #pragma unroll
         for (int i = 0; i < 9; i++) d[i] = f[i] - feq[i];
         if (!FIXED && exact_sums<9, 3>(f, feq, d)) {
+            if (__double2hiint(f[0]) > 0) hint = density_hint(rho, R);
             const double s56 = d[5] + d[6], s78 = d[7] + d[8], t = s56 + s78;
             pxx = (d[1] + d[2]) + t;
             pyy = (d[3] + d[4]) + t;
@@ -407,7 +423,7 @@ __device__ __forceinline__ void equilibrium19_int(double rho, double ux, double 
 }
 
 template <int OP, bool FIXED>
-__device__ __forceinline__ void collide19(double f[19], const Relax &R)
+__device__ __forceinline__ void collide19(double f[19], const Relax &R, uint32_t &hint)
 {
     double rho, ux, uy, uz, feq[19];
     int64_t F[19];
@@ -425,6 +441,7 @@ __device__ __forceinline__ void collide19(double f[19], const Relax &R)
     double d[19], pxx, pyy, pzz, pxy, pxz, pyz;
     int64_t D[19];
     if (fixed && fixed_parts<19, 4>(F, feq, D)) {
+        hint = density_hint(rho, R);
         const int64_t a = D[7] + D[8], b = D[9] + D[10], ab = a + b;
         const int64_t g = D[11] + D[12], h = D[13] + D[14], gh = g + h;
         const int64_t m = D[15] + D[16], n = D[17] + D[18], mn = m + n;
@@ -440,6 +457,7 @@ __device__ __forceinline__ void collide19(double f[19], const Relax &R)
 #pragma unroll
         for (int i = 0; i < 19; i++) d[i] = f[i] - feq[i];
         if (!FIXED && exact_sums<19, 4>(f, feq, d)) {
+            if (__double2hiint(f[0]) > 0) hint = density_hint(rho, R);
             const double a = d[7] + d[8], b = d[9] + d[10], ab = a + b;
             const double g = d[11] + d[12], h = d[13] + d[14], gh = g + h;
             const double m = d[15] + d[16], n = d[17] + d[18], mn = m + n;
@@ -489,13 +507,15 @@ __device__ __forceinline__ void collide19(double f[19], const Relax &R)
 }
 
 template <int Q, int OP, bool FIXED = true>
-__device__ __forceinline__ void collide(double *f, const Relax &R)
+__device__ __forceinline__ uint32_t collide(double *f, const Relax &R)
 {
     static_assert(Q == 9 || OP != OP_MRT, "MRT is a D2Q9 operator");
+    uint32_t hint = NO_HINT;
     if constexpr (Q == 9)
-        collide9<OP, FIXED>(f, R);
+        collide9<OP, FIXED>(f, R, hint);
     else
-        collide19<OP, FIXED>(f, R);
+        collide19<OP, FIXED>(f, R, hint);
+    return hint;
 }
 
 // calcula velocity of one node (for kinectic_energy, Other_functions.cpp:100-115):
@@ -525,37 +545,48 @@ __device__ __forceinline__ double node_density(const double *f)
 }
 
 // ZouHeD3Q19_vx_x, left-plane branch (Boundary_conditions.cpp:370-403) with vy = vz = 0, applied
-// to one node's post-stream populations.  The right-plane branch (:404-436) mirrors it.
-__device__ __forceinline__ void zou_he_left(double f[19], double vx)
+// to one node's post-stream populations.  The right-plane branch (:404-436) mirrors it.  The terms with
+// vy and vz are +-0; x / 6 is half of x / 3, so that 0.5 ty and rho vx / 6 enter by fused multiply-adds by exact
+// halves; a quotient by a constant of the run is fp64int::quotient.  About 50 FP64 operations instead of 90.
+struct ZouHe {
+    double vx, y, z;  // y = 1 - vx; z = 1 / y, or 0 where no reciprocal was formed
+};
+
+__device__ __forceinline__ double zou_he_quotient(double a, const ZouHe &c)
 {
-    const double vy = 0.0, vz = 0.0;
-    const double s_minus = (((f[1] + f[7]) + f[9]) + f[11]) + f[13];
-    const double s_zero = (((((((f[0] + f[3]) + f[4]) + f[5]) + f[6]) + f[15]) + f[16]) + f[17]) + f[18];
-    const double rho = (2.0 * s_minus + s_zero) / (1.0 - vx);
-    const double ty = (((((f[18] + f[3]) + f[16]) - f[15]) - f[4]) - f[17]);
-    const double tz = (((((f[17] + f[5]) + f[16]) - f[15]) - f[6]) - f[18]);
-    const double a3 = rho * vx / 3.0, a6 = rho * vx / 6.0;
-    f[1] = f[1] + a3;
-    f[7] = ((f[7] + a6) + 0.5 * rho * vy) - 0.5 * ty;
-    f[9] = ((f[9] + a6) - 0.5 * rho * vy) + 0.5 * ty;
-    f[11] = ((f[11] + a6) + 0.5 * rho * vz) - 0.5 * tz;
-    f[13] = ((f[13] + a6) - 0.5 * rho * vz) + 0.5 * tz;
+    return c.z != 0.0 && fp64int::quotient_range(a) ? fp64int::quotient(a, c.y, c.z) : a / c.y;
 }
 
-__device__ __forceinline__ void zou_he_right(double f[19], double vx)
+__device__ __forceinline__ double third(double a) { return fp64int::quotient_range(a) ? fp64int::quotient3(a) : a / 3.0; }
+
+__device__ __forceinline__ void zou_he_left(double f[19], const ZouHe &c)
 {
-    const double vy = 0.0, vz = 0.0;
-    const double s_plus = (((f[2] + f[8]) + f[10]) + f[12]) + f[14];
+    const double s_minus = (((f[1] + f[7]) + f[9]) + f[11]) + f[13];
     const double s_zero = (((((((f[0] + f[3]) + f[4]) + f[5]) + f[6]) + f[15]) + f[16]) + f[17]) + f[18];
-    const double rho = (2.0 * s_plus + s_zero) / (1.0 - vx);
+    const double rho = zou_he_quotient(__fma_rn(2.0, s_minus, s_zero), c);
     const double ty = (((((f[18] + f[3]) + f[16]) - f[15]) - f[4]) - f[17]);
     const double tz = (((((f[17] + f[5]) + f[16]) - f[15]) - f[6]) - f[18]);
-    const double a3 = rho * vx / 3.0, a6 = rho * vx / 6.0;
+    const double a3 = third(rho * c.vx);
+    f[1] = f[1] + a3;
+    f[7] = __fma_rn(-0.5, ty, __fma_rn(0.5, a3, f[7]));
+    f[9] = __fma_rn(0.5, ty, __fma_rn(0.5, a3, f[9]));
+    f[11] = __fma_rn(-0.5, tz, __fma_rn(0.5, a3, f[11]));
+    f[13] = __fma_rn(0.5, tz, __fma_rn(0.5, a3, f[13]));
+}
+
+__device__ __forceinline__ void zou_he_right(double f[19], const ZouHe &c)
+{
+    const double s_plus = (((f[2] + f[8]) + f[10]) + f[12]) + f[14];
+    const double s_zero = (((((((f[0] + f[3]) + f[4]) + f[5]) + f[6]) + f[15]) + f[16]) + f[17]) + f[18];
+    const double rho = zou_he_quotient(__fma_rn(2.0, s_plus, s_zero), c);
+    const double ty = (((((f[18] + f[3]) + f[16]) - f[15]) - f[4]) - f[17]);
+    const double tz = (((((f[17] + f[5]) + f[16]) - f[15]) - f[6]) - f[18]);
+    const double a3 = third(rho * c.vx);
     f[2] = f[2] - a3;
-    f[10] = ((f[10] - a6) + 0.5 * rho * vy) - 0.5 * ty;
-    f[8] = ((f[8] - a6) - 0.5 * rho * vy) + 0.5 * ty;
-    f[14] = ((f[14] - a6) + 0.5 * rho * vz) - 0.5 * tz;
-    f[12] = ((f[12] - a6) - 0.5 * rho * vz) + 0.5 * tz;
+    f[10] = __fma_rn(-0.5, ty, __fma_rn(-0.5, a3, f[10]));
+    f[8] = __fma_rn(0.5, ty, __fma_rn(-0.5, a3, f[8]));
+    f[14] = __fma_rn(-0.5, tz, __fma_rn(-0.5, a3, f[14]));
+    f[12] = __fma_rn(0.5, tz, __fma_rn(-0.5, a3, f[12]));
 }
 
 // ZouHeD2Q9_vx_x (Boundary_conditions.cpp:710-744), also the node update of parabolic_D2Q9_x

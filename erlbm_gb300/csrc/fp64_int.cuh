@@ -106,6 +106,35 @@ __host__ __device__ __forceinline__ void eq_pair(double cv, double cv2, uint64_t
     minus = from_bits(neg ? up : uq);
 }
 
+// ---- quotients by a constant ------------------------------------------------------------------------------------
+// a / y rounded to nearest from z = RN(1 / y): a quotient within an ulp corrected by one fused step on its exact
+// residual (Markstein's theorem, which asks for a correctly rounded reciprocal), after one step that brings the
+// product a z within an ulp.  For |a| and |y| well inside the exponent range.  5 operations.
+__host__ __device__ __forceinline__ double fused(double a, double b, double c)
+{
+#ifdef __CUDA_ARCH__
+    return __fma_rn(a, b, c);
+#else
+    return __builtin_fma(a, b, c);
+#endif
+}
+__host__ __device__ __forceinline__ bool quotient_range(double a)
+{
+    return (hi32(bits(a)) & 0x7fffffffu) - 0x20000000u < 0x3ff00000u;  // 2^-511 <= |a| < 2^512
+}
+__host__ __device__ __forceinline__ double quotient(double a, double y, double z)
+{
+    double q = a * z;
+    q = fused(fused(-y, q, a), z, q);
+    return fused(fused(-y, q, a), z, q);
+}
+// a / 3: RN(1/3) is a quarter ulp off, so that a z is within an ulp at once.  3 operations.
+__host__ __device__ __forceinline__ double quotient3(double a)
+{
+    const double z = 1.0 / 3.0, q = a * z;
+    return fused(fused(-3.0, q, a), z, q);
+}
+
 // ---- populations in fixed point --------------------------------------------------------------------------------
 // A population 2^-6 <= f < 1 is a whole number of units of 2^-58 below 2^58.
 

@@ -39,6 +39,12 @@ struct PrecExact64 {
     {
         exact::collide<Q, OP>(f, p.R);
     }
+    // The collision, returning exact::density_hint of the node
+    template <int Q, int OP>
+    __device__ static __forceinline__ uint32_t collide_hint(T *f, const CollParams &p)
+    {
+        return exact::collide<Q, OP>(f, p.R);
+    }
     template <int Q>
     __device__ static __forceinline__ double density(const T *f)
     {
@@ -61,16 +67,20 @@ struct PrecExact64 {
         }
     }
     // Zou-He closure constants of one inlet velocity: the exact path uses vx as the reference does
-    struct ZouHe {
-        double vx;
-    };
-    __device__ static __forceinline__ ZouHe zou_he_prep(double vx) { return ZouHe{vx}; }
+    using ZouHe = exact::ZouHe;
+    __device__ static __forceinline__ ZouHe zou_he_prep(double vx) { return ZouHe{vx, 1.0 - vx, 0.0}; }
+    // for a whole run, with the reciprocal of 1 - vx where quotients by it stay in range
+    __device__ static __forceinline__ ZouHe zou_he_prep_run(double vx)
+    {
+        const double y = 1.0 - vx, a = fabs(y);
+        return ZouHe{vx, y, a > 0x1p-100 && a < 0x1p100 ? 1.0 / y : 0.0};
+    }
     __device__ static __forceinline__ void zou_he(T *f, const ZouHe &z, bool left)
     {
         if (left)
-            exact::zou_he_left(f, z.vx);
+            exact::zou_he_left(f, z);
         else
-            exact::zou_he_right(f, z.vx);
+            exact::zou_he_right(f, z);
     }
     // ZouHeD2Q9_vx_x, and the node update of parabolic_D2Q9_x / parabolic_D3Q19_x with a profile velocity
     __device__ static __forceinline__ void zou_he9(T *f, double vx) { exact::zou_he_d2q9(f, vx); }
@@ -122,6 +132,11 @@ struct PrecExact64Small : PrecExact64 {
     {
         exact::collide<Q, OP, false>(f, p.R);
     }
+    template <int Q, int OP>
+    __device__ static __forceinline__ uint32_t collide_hint(T *f, const CollParams &p)
+    {
+        return exact::collide<Q, OP, false>(f, p.R);
+    }
 };
 
 struct PrecShifted32 {
@@ -130,6 +145,12 @@ struct PrecShifted32 {
     __device__ static __forceinline__ void collide(T *f, const CollParams &p)
     {
         shifted::collide<Q, OP>(f, p.k);
+    }
+    template <int Q, int OP>
+    __device__ static __forceinline__ uint32_t collide_hint(T *f, const CollParams &p)
+    {
+        shifted::collide<Q, OP>(f, p.k);
+        return exact::NO_HINT;
     }
     template <int Q>
     __device__ static __forceinline__ double density(const T *f)
@@ -156,6 +177,7 @@ struct PrecShifted32 {
     }
     using ZouHe = shifted::ZouHe;
     __device__ static __forceinline__ ZouHe zou_he_prep(double vx) { return shifted::zou_he_prep(vx); }
+    __device__ static __forceinline__ ZouHe zou_he_prep_run(double vx) { return shifted::zou_he_prep(vx); }
     __device__ static __forceinline__ void zou_he(T *f, const ZouHe &z, bool left) { shifted::zou_he(f, z, left); }
     __device__ static __forceinline__ void zou_he9(T *f, double vx) { shifted::zou_he_d2q9(f, vx); }
     template <int Q>
@@ -379,21 +401,22 @@ __device__ void state_after_planes(const typename P::T *__restrict__ src, const 
 // ------------------------------------------------------------------------------------------------
 
 // One node of one step: state after the planes, collision, the density check, store.  rho_bits and
-// flag return the check's outcome (|rho| as a bit pattern; 1 above the limit, 2 non-finite).  The body
+// flag return the check's outcome (|rho| as a bit pattern; 1 above the limit, 2 non-finite).  known: the upper word
+// of a density the check has seen; a node whose density is certainly below it returns 0.  The body
 // of k_step, shared with the resident team loop so that both give the same bits.
 template <class P, int Q, int OP, bool COH = false>
 __device__ __forceinline__ void step_node(const typename P::T *__restrict__ src, typename P::T *__restrict__ dst,
                                           const Geo &g, const BCp &bc, const CollParams &prm, int mode,
                                           int check_density, double density_limit, long long node,
-                                          unsigned long long &rho_bits, int &flag)
+                                          unsigned long long &rho_bits, int &flag, uint32_t known = 0)
 {
     using T = typename P::T;
     int x, y, z;
     node_xyz(g, node, x, y, z);
     T f[Q];
     state_after_planes<P, Q, COH>(src, g, bc, mode, x, y, z, node, f);
-    P::template collide<Q, OP>(f, prm);
-    if (check_density) {
+    const uint32_t hint = P::template collide_hint<Q, OP>(f, prm);
+    if (check_density && !exact::density_below(hint, known)) {
         const double rho = P::template density<Q>(f);
         if (!isfinite(rho)) {
             flag = 2;
@@ -411,6 +434,7 @@ __device__ __forceinline__ void step_node(const typename P::T *__restrict__ src,
 // lane of the warp calls it.
 __device__ __forceinline__ void report_density(RunStatus *status, int step_index, unsigned long long rho_bits, int flag)
 {
+    if (!__any_sync(0xffffffffu, rho_bits != 0 || flag != 0)) return;
     const unsigned long long m = warp_max_u64(rho_bits);
     const int any = __reduce_or_sync(0xffffffffu, flag);
     if ((threadIdx.x & 31) == 0) {
@@ -439,8 +463,10 @@ __global__ void __launch_bounds__(256) k_step(const typename P::T *__restrict__ 
     if (active && g.solid != nullptr && g.solid[node]) active = false;
     unsigned long long rho_bits = 0;
     int flag = 0;
+    uint32_t known = 0;  // read while the populations are
+    if (a.check_density) known = (uint32_t)(*(volatile unsigned long long *)&a.status->max_abs_rho_bits >> 32);
     if (active)
-        step_node<P, Q, OP>(src, dst, g, bc, prm, a.mode, a.check_density, a.density_limit, node, rho_bits, flag);
+        step_node<P, Q, OP>(src, dst, g, bc, prm, a.mode, a.check_density, a.density_limit, node, rho_bits, flag, known);
     if (a.check_density) report_density(a.status, a.step_index, rho_bits, flag);
 }
 

@@ -171,7 +171,7 @@ extern "C" int erlbm_batch_run_noalloc(const erlbm_batch_desc *d, int n_runs, co
     memset(&g, 0, sizeof(g));
     g.nx = d->nx;
     g.ny = d->ny;
-    g.nb = d->nx * d->ny;
+    g.nb = g.n_fluid = d->nx * d->ny;
     g.solid = d->solid;  // a device pointer here
     g.inlet_x = d->inlet_x;
     g.outlet_x = d->outlet_x;

@@ -60,6 +60,18 @@ int main(int argc, char **argv)
             cases++;
         }
     }
+    // quotients by a constant and by 3
+    for (long it = 0; it < n; it++) {
+        const double y = std::ldexp(1.0 + std::ldexp((double)(rng() >> 12), -52), (int)(rng() % 9) - 6);
+        double a = std::ldexp((double)(int64_t)rng(), -(int)(rng() % 600));
+        if (rng() % 3 == 0) a = y * (double)(1 + rng() % 64) * (1.0 + std::ldexp((double)(rng() % 5) - 2.0, -52));
+        if (!quotient_range(a)) continue;
+        cases++;
+        bad += bits(quotient(a, y, 1.0 / y)) != bits(a / y) || bits(quotient3(a)) != bits(a / 3.0);
+    }
+    for (double x : {0.0, -0.0, 0x1p-1022, 0x1p-512, 0x1p512, 0x1p1023, (double)INFINITY, (double)NAN})
+        bad += quotient_range(x) || quotient_range(-x);
+    bad += !quotient_range(0x1p-511) || !quotient_range(-1.0) || !quotient_range(0x1.8p511);
     const double out[] = {1.0, 1.5, 0x1p-7, 0x1.fffffffffffffp-7, -0.1, 0.0, -0.0, INFINITY, -INFINITY, NAN};
     for (double x : out) bad += fix_range(x) < FIX_SPAN;
     printf("%ld %ld\n", cases, bad);
