@@ -129,7 +129,7 @@ __device__ __forceinline__ bool fixed_form(const double *f)
     uint32_t most = 0;
 #pragma unroll
     for (int i = 0; i < Q; i++) most = max(most, fp64int::fix_range(f[i]));
-    return most < fp64int::FIX_SPAN;
+    return most < (Q == 9 ? fp64int::FIX_SPAN : fp64int::FIX_SPAN_HALF);
 }
 
 // moments9 with its sums in fixed point (fixed_form holds), every partial sum rounded as the FP64 add rounds it:
@@ -151,10 +151,13 @@ __device__ __forceinline__ void moments9_fixed(const double f[9], int64_t F[9], 
     uy = fp64int::to_double(my) * inv;
 }
 
-// D_i = f_i - feq_i in fixed point.  True when every feq has the fixed-point form too and every |D_i| < 2^(53 - M):
-// then each D_i is exact, and so is every sum of up to 2^M of them in any order.
-template <int Q, int M>
-__device__ __forceinline__ bool fixed_parts(const int64_t *F, const double *feq, int64_t *D)
+// D_i = f_i - feq_i in fixed point, exact.  False when a feq has no fixed-point form.  shared: every |D_i| is small
+// enough that sums of up to 10 of them (6 for nine populations) stay below 2^53 units: then the D_i are FP64 numbers,
+// and their sums are exact in any order, so that the terms the sums share are added once.  Otherwise D_i is rounded as
+// the FP64 difference is, and so is every partial sum in the reference's order (low viscosity: most nodes of the
+// obstacle map's lower rows; those took 55 FP64 operations more).
+template <int Q>
+__device__ __forceinline__ bool fixed_parts(const int64_t *F, const double *feq, int64_t *D, bool &shared)
 {
     if (!fixed_form<Q>(feq)) return false;
     uint32_t most = 0;
@@ -162,9 +165,23 @@ __device__ __forceinline__ bool fixed_parts(const int64_t *F, const double *feq,
     for (int i = 0; i < Q; i++) {
         D[i] = F[i] - fp64int::to_fixed(feq[i]);
         const int32_t h = (int32_t)fp64int::hi32((uint64_t)D[i]);
-        most |= (uint32_t)(h ^ (h >> 31));
+        most = max(most, (uint32_t)(h ^ (h >> 31)));
     }
-    return most < (1u << (21 - M));
+    shared = most < (1u << 21) / (Q == 9 ? 6 : 10) - 1;
+    if (!shared) {
+#pragma unroll
+        for (int i = 0; i < Q; i++) D[i] = fp64int::round53(D[i]);
+    }
+    return true;
+}
+
+// D[I0] + D[I] + ... in order, every sum rounded; a negative index -I stands for - D[I].
+template <int I0, int... I>
+__device__ __forceinline__ int64_t rounded_sum(const int64_t *D)
+{
+    int64_t s = D[I0];
+    ((s = fp64int::round53(I > 0 ? s + D[I > 0 ? I : -I] : s - D[I > 0 ? I : -I])), ...);
+    return s;
 }
 
 // Row ROW of the MRT transform applied to f: the reference sums M[ROW][i] * f[i] from 0.0 in
@@ -286,12 +303,23 @@ __device__ __forceinline__ void collide9(double f[9], const Relax &R, uint32_t &
     }
     double d[9], pxx, pyy, pxy;
     int64_t D[9];
-    if (fixed && fixed_parts<9, 3>(F, feq, D)) {
+    bool shared;
+    if (fixed && fixed_parts<9>(F, feq, D, shared)) {
         hint = density_hint(rho, R);
-        const int64_t s56 = D[5] + D[6], s78 = D[7] + D[8], t = s56 + s78;
-        pxx = fp64int::to_double((D[1] + D[2]) + t);
-        pyy = fp64int::to_double((D[3] + D[4]) + t);
-        pxy = fp64int::to_double(s56 - s78);
+        int64_t xx, yy, xy;
+        if (shared) {
+            const int64_t s56 = D[5] + D[6], s78 = D[7] + D[8], t = s56 + s78;
+            xx = (D[1] + D[2]) + t;
+            yy = (D[3] + D[4]) + t;
+            xy = s56 - s78;
+        } else {
+            xx = rounded_sum<1, 2, 5, 6, 7, 8>(D);
+            yy = rounded_sum<3, 4, 5, 6, 7, 8>(D);
+            xy = rounded_sum<5, 6, -7, -8>(D);
+        }
+        pxx = fp64int::to_double(xx);
+        pyy = fp64int::to_double(yy);
+        pxy = fp64int::to_double(xy);
 #pragma unroll
         for (int i = 0; i < 9; i++) d[i] = fp64int::to_double(D[i]);
     } else {
@@ -440,17 +468,34 @@ __device__ __forceinline__ void collide19(double f[19], const Relax &R, uint32_t
     }
     double d[19], pxx, pyy, pzz, pxy, pxz, pyz;
     int64_t D[19];
-    if (fixed && fixed_parts<19, 4>(F, feq, D)) {
+    bool shared;
+    if (fixed && fixed_parts<19>(F, feq, D, shared)) {
         hint = density_hint(rho, R);
-        const int64_t a = D[7] + D[8], b = D[9] + D[10], ab = a + b;
-        const int64_t g = D[11] + D[12], h = D[13] + D[14], gh = g + h;
-        const int64_t m = D[15] + D[16], n = D[17] + D[18], mn = m + n;
-        pxx = fp64int::to_double((D[1] + D[2]) + (ab + gh));
-        pyy = fp64int::to_double((D[3] + D[4]) + (ab + mn));
-        pzz = fp64int::to_double((D[5] + D[6]) + (gh + mn));
-        pxy = fp64int::to_double(a - b);
-        pxz = fp64int::to_double(g - h);
-        pyz = fp64int::to_double(m - n);
+        int64_t xx, yy, zz, xy, xz, yz;
+        if (shared) {
+            const int64_t a = D[7] + D[8], b = D[9] + D[10], ab = a + b;
+            const int64_t g = D[11] + D[12], h = D[13] + D[14], gh = g + h;
+            const int64_t m = D[15] + D[16], n = D[17] + D[18], mn = m + n;
+            xx = (D[1] + D[2]) + (ab + gh);
+            yy = (D[3] + D[4]) + (ab + mn);
+            zz = (D[5] + D[6]) + (gh + mn);
+            xy = a - b;
+            xz = g - h;
+            yz = m - n;
+        } else {
+            xx = rounded_sum<1, 2, 7, 8, 9, 10, 11, 12, 13, 14>(D);
+            yy = rounded_sum<3, 4, 7, 8, 9, 10, 15, 16, 17, 18>(D);
+            zz = rounded_sum<5, 6, 11, 12, 13, 14, 15, 16, 17, 18>(D);
+            xy = rounded_sum<7, 8, -9, -10>(D);
+            xz = rounded_sum<11, 12, -13, -14>(D);
+            yz = rounded_sum<15, 16, -17, -18>(D);
+        }
+        pxx = fp64int::to_double(xx);
+        pyy = fp64int::to_double(yy);
+        pzz = fp64int::to_double(zz);
+        pxy = fp64int::to_double(xy);
+        pxz = fp64int::to_double(xz);
+        pyz = fp64int::to_double(yz);
 #pragma unroll
         for (int i = 0; i < 19; i++) d[i] = fp64int::to_double(D[i]);
     } else {

@@ -136,12 +136,13 @@ __host__ __device__ __forceinline__ double quotient3(double a)
 }
 
 // ---- populations in fixed point --------------------------------------------------------------------------------
-// A population 2^-6 <= f < 1 is a whole number of units of 2^-58 below 2^58.
+// A population 2^-7 <= f < 1 is a whole number of units of 2^-59 below 2^59.
 
-constexpr int FIX_E0 = 1017;  // exponent field of 2^-6
+constexpr int FIX_E0 = 1016;  // exponent field of 2^-7
 
-// max over values of this is below FIX_SPAN when all of them are in range (negative ones and NaN are not)
-constexpr uint32_t FIX_SPAN = 6u << 20;
+// max over values of fix_range is below this when all of them are in range (negative ones and NaN are not): up to 1
+// for nine populations, up to 1/2 for nineteen, so that their sum stays below 2^63 units
+constexpr uint32_t FIX_SPAN = 7u << 20, FIX_SPAN_HALF = 6u << 20;
 __host__ __device__ __forceinline__ uint32_t fix_range(double f) { return hi32(bits(f)) - ((uint32_t)FIX_E0 << 20); }
 
 __host__ __device__ __forceinline__ int64_t to_fixed(double f)
@@ -167,7 +168,7 @@ __host__ __device__ __forceinline__ int clz64(uint64_t x)
 #endif
 }
 
-// x rounded to 53 significant bits, ties to even (|x| < 2^62).  Rounding by the floor of x + half works on
+// x rounded to 53 significant bits, ties to even (|x| < 2^63).  Rounding by the floor of x + half works on
 // two's complement as it is; the magnitude's leading bit is found on x or its complement.
 __host__ __device__ __forceinline__ int64_t round53(int64_t x)
 {
@@ -185,7 +186,7 @@ __host__ __device__ __forceinline__ double to_double(int64_t x)
     const uint64_t a = x < 0 ? 0 - (uint64_t)x : (uint64_t)x;
     const int lz = clz64(a) & 63;
     const uint64_t m = (a << lz) >> 11;  // leading bit at 52: it adds 1 to the exponent field
-    const uint64_t b = m + ((uint64_t)(uint32_t)(1027 - lz) << 52);
+    const uint64_t b = m + ((uint64_t)(uint32_t)(1026 - lz) << 52);
     return from_bits(a == 0 ? 0 : b | ((uint64_t)x & 0x8000000000000000ull));
 }
 
