@@ -1,18 +1,99 @@
 // k_fp64.cu -- plain FP64 kernels.  This translation unit is compiled with --fmad=false so that
 // every multiply and add is rounded on its own, as in the reference's GCC -std=c++17 build.
 #include "lattice_kernels.cuh"
+#include "quad_fp64.cuh"
 
 namespace erlbm {
 
-// From this size on every scheduler has two warps or more, and the fixed-point sums of the collision cost
+// From this size on (past QUAD_MAX_NODES: the small sizes below are those of one lane a node) every scheduler has two
+// warps or more, and the fixed-point sums of the collision cost
 // less than the FP64 operations they replace; below, a warp waits for its own integer chains.  us per step without
 // and with: D3Q19 16^3 14.4 / 18.5, 24^3 15.4 / 18.5, 32^3 23.7 / 22.6, 64^3 135.7 / 114.9; D2Q9 160^2 10.3 / 10.3,
 // 200^2 16.3 / 13.4, 512^2 65.7 / 49.2.
 constexpr long long FIXED_MIN_NODES = 32768;
 
+namespace {
+
+// k_step with four lanes a node (quad_fp64.cuh).
+constexpr int QUAD_BLOCK = 64;
+
+template <int Q, int OP>
+__global__ void __launch_bounds__(QUAD_BLOCK) k_step_quad(const double *__restrict__ src, double *__restrict__ dst, Geo g,
+                                                          BCp bc, Relax R, StepArgs a)
+{
+    after_previous();
+    if (a.stop_on_flag && a.status != nullptr) {  // as k_step
+        const int ds = __shfl_sync(0xffffffffu, *(volatile int *)&a.status->decided_step, 0);
+        if (ds < a.step_index) return;
+    }
+    uint32_t known = 0;
+    if (a.check_density) known = (uint32_t)(*(volatile unsigned long long *)&a.status->max_abs_rho_bits >> 32);
+    const unsigned thread = blockIdx.x * QUAD_BLOCK + threadIdx.x;
+    const long long node = thread >> 2;
+    const quad::Team t{(int)(threadIdx.x & 3), (int)(threadIdx.x & 28)};
+    bool active = node < g.nbox;
+    if (active && g.solid != nullptr && g.solid[node]) active = false;
+    double f[Q], out[2 * quad::SLOTS<Q>];
+    if (active) {
+        int x, y, z;
+        node_xyz(g, node, x, y, z);
+        state_after_planes<PrecExact64, Q>(src, g, bc, a.mode, x, y, z, node, f);
+    } else {  // lanes without a node take part in the warp's shuffles
+#pragma unroll
+        for (int i = 0; i < Q; i++) f[i] = Lat<Q>::w(i);
+    }
+    const uint32_t hint = quad::collide<Q, OP>(f, t, R, out);
+    if (active) {
+#pragma unroll
+        for (int k = 0; k < 2 * quad::SLOTS<Q>; k++) {
+            const int i = quad::population<Q>(t.sub, k / 2, k % 2);
+            if (i >= 0) dst[(long long)i * g.plane + node] = out[k];
+        }
+    }
+    if (!a.check_density) return;
+    const bool check = active && !exact::density_below(hint, known);
+    if (!__any_sync(0xffffffffu, check)) return;
+    double p[Q];
+#pragma unroll
+    for (int i = 0; i < Q; i++) p[i] = quad::gathered<Q>(out, t, i);
+    const double rho = exact::node_density<Q>(p);
+    unsigned long long rho_bits = 0;
+    int flag = 0;
+    if (check && !isfinite(rho)) {
+        flag = 2;
+    } else if (check) {
+        rho_bits = (unsigned long long)__double_as_longlong(fabs(rho));
+        if (fabs(rho) > a.density_limit) flag = 1;
+    }
+    report_density(a.status, a.step_index, rho_bits, flag);
+}
+
+// Four lanes a node up to this size.  4864 nodes give each of the 608 schedulers one such warp; beyond, a second warp
+// shares the FP64 pipe, and the 13.6 warp instructions a node (8 for one lane a node) decide.  us per step with one
+// lane and with four: D2Q9 32^2 6.3 / 4.4, 64^2 6.3 / 4.5, 90^2 6.3 / 6.4, 112^2 6.8 / 8.6; D3Q19 10^3 12.6 / 6.7, 16^3
+// 12.3 / 7.1, 20^3 12.3 / 10.4, 22^3 13.2 / 14.4; 82 x 48 D3Q19 with planes and solids 12.3 / 7.1.
+template <int Q>
+constexpr long long QUAD_MAX_NODES = Q == 9 ? 7296 : 9728;
+
+template <int Q, int OP>
+int launch_quad(const Geo &g, const BCp &bc, const Relax &R, const StepArgs &a, const double *src, double *dst,
+                cudaStream_t s)
+{
+    launch_step_kernel<k_step_quad<Q, OP>, QUAD_BLOCK>(blocks_for(4 * g.nbox, QUAD_BLOCK), s, src, dst, g, bc, R, a);
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+}
+
+}  // namespace
+
 int launch_step_fp64(int q, int op, const Geo &g, const BCp &bc, const Relax &R, const StepArgs &a, const double *src,
                      double *dst, cudaStream_t s)
 {
+    if ((q == 9 && g.nbox <= QUAD_MAX_NODES<9>) || (q == 19 && g.nbox <= QUAD_MAX_NODES<19>)) {
+        if (op == OP_BGK) return (q == 9 ? launch_quad<9, OP_BGK> : launch_quad<19, OP_BGK>)(g, bc, R, a, src, dst, s);
+        if (op == OP_REG) return (q == 9 ? launch_quad<9, OP_REG> : launch_quad<19, OP_REG>)(g, bc, R, a, src, dst, s);
+        if (op == OP_EXTREG)
+            return (q == 9 ? launch_quad<9, OP_EXTREG> : launch_quad<19, OP_EXTREG>)(g, bc, R, a, src, dst, s);
+    }
     if (g.nbox < FIXED_MIN_NODES) return step_any<PrecExact64Small>(q, op, g, bc, R, a, src, dst, s);
     return step_any<PrecExact64>(q, op, g, bc, R, a, src, dst, s);
 }

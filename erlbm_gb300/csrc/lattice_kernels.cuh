@@ -124,7 +124,7 @@ struct PrecExact64 {
     __device__ static __forceinline__ double to_f(T v, int) { return v; }
 };
 
-// The exact path for lattices of fewer warps than hide the latency of the fixed-point sums: the same bits with
+// The exact path for MRT lattices and lattices past four lanes a node (k_fp64.cu) of fewer warps than hide the latency of the fixed-point sums: the same bits with
 // more FP64 operations and fewer dependent integer ones.
 struct PrecExact64Small : PrecExact64 {
     template <int Q, int OP>

@@ -74,3 +74,24 @@ def test_fp64_collision_at_the_limits_of_the_integer_forms(q, shape, op, kind):
         want = ref.get(1)
         fine = np.isfinite(want)
         assert np.array_equal(np.isfinite(got), fine) and np.array_equal(got[fine], want[fine])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("q,shape", [(9, (131, 83, 1)), (9, (211, 157, 1)), (19, (29, 23, 17)), (19, (41, 32, 26))])
+@pytest.mark.parametrize("kind", ["rest", "mach", "dense", "noise", "dyadic", "holes"])
+def test_fp64_collision_of_larger_lattices(q, shape, kind):
+    """The same for lattices past the sizes of four lanes a node, and past those of FP64 sums."""
+    import erlbm_gb300 as E
+    n = int(np.prod(shape))
+    f = states(q, n, kind, np.random.default_rng(n))
+    for op in (3, 4):
+        ref = O.Lattice(q, *shape, None, 0.52, 0.65, op)
+        ref.set(f)
+        ref.step(3)
+        with E.Lattice(q, *shape, None, 0.52, 0.65, op, E.FP64) as lat:
+            lat.set_populations(f)
+            lat.step(3)
+            got = lat.get_populations(E.STAGE_POST_COLLISION)
+        want = ref.get(1)
+        fine = np.isfinite(want)
+        assert np.array_equal(np.isfinite(got), fine) and np.array_equal(got[fine], want[fine])
