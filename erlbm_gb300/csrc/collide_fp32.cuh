@@ -118,6 +118,14 @@ struct LaneF1 {
     static __device__ __forceinline__ V fma(V a, V b, V d) { return __fmaf_rn(a, b, d); }
     static __device__ __forceinline__ V neg(V a) { return -a; }
     static __device__ __forceinline__ V rcp(V a) { return rcp_rn(a); }
+    // x a and x a + d for a float x; x a + d and -x a + d; the same for a power of two x: forms that a wider lane
+    // has for less
+    static __device__ __forceinline__ V mulc(float x, V a) { return mul(c(x), a); }
+    static __device__ __forceinline__ V fmac(float x, V a, V d) { return fma(c(x), a, d); }
+    static __device__ __forceinline__ V fma2p(float x, V a, V d) { return fma(c(x), a, d); }
+    static __device__ __forceinline__ void fma_pm(V x, V a, V d, V &p, V &m) { p = fma(x, a, d), m = fma(neg(x), a, d); }
+    static __device__ __forceinline__ void fmac_pm(float x, V a, V d, V &p, V &m) { fma_pm(c(x), a, d, p, m); }
+    static __device__ __forceinline__ void fma2p_pm(float x, V a, V d, V &p, V &m) { fma_pm(c(x), a, d, p, m); }
 };
 
 struct LaneF2 {
@@ -130,6 +138,12 @@ struct LaneF2 {
     static __device__ __forceinline__ V mul(V a, V b) { return __fmul2_rn(a, b); }
     static __device__ __forceinline__ V fma(V a, V b, V d) { return __ffma2_rn(a, b, d); }
     static __device__ __forceinline__ V neg(V a) { return make_float2(-a.x, -a.y); }
+    static __device__ __forceinline__ V mulc(float x, V a) { return mul(c(x), a); }
+    static __device__ __forceinline__ V fmac(float x, V a, V d) { return fma(c(x), a, d); }
+    static __device__ __forceinline__ V fma2p(float x, V a, V d) { return fma(c(x), a, d); }
+    static __device__ __forceinline__ void fma_pm(V x, V a, V d, V &p, V &m) { p = fma(x, a, d), m = fma(neg(x), a, d); }
+    static __device__ __forceinline__ void fmac_pm(float x, V a, V d, V &p, V &m) { fma_pm(c(x), a, d, p, m); }
+    static __device__ __forceinline__ void fma2p_pm(float x, V a, V d, V &p, V &m) { fma_pm(c(x), a, d, p, m); }
     // rcp_rn on both halves: one range test for the pair, the correction step in packed form
     static __device__ __forceinline__ V rcp(V a)
     {
@@ -162,8 +176,10 @@ __device__ __forceinline__ void update_pair2_l(typename M::V &gi, typename M::V 
         // every product here feeds an explicit fma, so there is nothing left for contraction to fuse
         const V kh = M::ck(k.kh);
         const V cm = M::fma(d1, f1, M::fma(M::ck(k.nkc), f1, M::mul(kh, D)));
-        gi = M::add(gi, M::fma(kh, DO, cm));
-        gj = M::add(gj, M::fma(M::neg(kh), DO, cm));
+        V ui, uj;
+        M::fma_pm(kh, DO, cm, ui, uj);
+        gi = M::add(gi, ui);
+        gj = M::add(gj, uj);
     }
 }
 
@@ -200,16 +216,18 @@ __device__ __forceinline__ void collide9l(typename M::V g[9], const K &k)
     // c = m_x u_y + m_y u_x: 4.5 a - 1.5 (a + b) on the x axis, 3 (a + b) +- 4.5 c on the diagonals
     const V a = M::mul(mx, ux), b = M::mul(my, uy);
     const V sab = M::fma(mx, ux, b);  // a + b as one rounding (no product is left to an add)
-    const V mu15 = M::mul(M::c(-1.5f), sab);
+    const V mu15 = M::mulc(-1.5f, sab);
     const V cxy = M::fma(mx, uy, M::mul(my, ux));
-    const V s3 = M::mul(M::c(3.f), sab);
-    const V k45 = M::c(4.5f), mw1x2 = M::kc(-2.f * W1, -2.0 / 9.0), mw2x2 = M::kc(-2.f * W2, -2.0 / 36.0);
+    const V s3 = M::mulc(3.f, sab);
+    V sP3, sM3;
+    M::fmac_pm(4.5f, cxy, s3, sP3, sM3);
+    const V mw1x2 = M::kc(-2.f * W1, -2.0 / 9.0), mw2x2 = M::kc(-2.f * W2, -2.0 / 36.0);
     // twice the even non-equilibrium parts
-    const V DX = M::fma(mw1x2, M::fma(k45, a, mu15), M::fma(mw1x2, drho, EX));
-    const V DY = M::fma(mw1x2, M::fma(k45, b, mu15), M::fma(mw1x2, drho, EY));
+    const V DX = M::fma(mw1x2, M::fmac(4.5f, a, mu15), M::fma(mw1x2, drho, EX));
+    const V DY = M::fma(mw1x2, M::fmac(4.5f, b, mu15), M::fma(mw1x2, drho, EY));
     const V cmP = M::add(mx, my), cmM = M::sub(mx, my);
-    const V DP = M::fma(mw2x2, M::fma(k45, cxy, s3), M::fma(mw2x2, drho, EP));
-    const V DM = M::fma(mw2x2, M::fma(M::c(-4.5f), cxy, s3), M::fma(mw2x2, drho, EM));
+    const V DP = M::fma(mw2x2, sP3, M::fma(mw2x2, drho, EP));
+    const V DM = M::fma(mw2x2, sM3, M::fma(mw2x2, drho, EM));
     // twice the odd non-equilibrium parts; the axis pairs close the momentum
     const V DOP = M::fma(M::kc(2.f * M3W2, -1.0 / 6.0), cmP, OP_);
     const V DOM = M::fma(M::kc(2.f * M3W2, -1.0 / 6.0), cmM, OM);
@@ -254,14 +272,13 @@ __device__ __forceinline__ void collide9l(typename M::V g[9], const K &k)
     // pxx - pyy = D_X - D_Y, the rest population's closure de0 = -(sxy + sd); f1 (f1X = pxx / 3 -
     // pyy / 6 written as (pxx - pyy) / 4 + tr / 12; f1_0 = -2/3 tr enters through d1t and nkct)
     const V sxy = M::add(DX, DY), sd = M::add(DP, DM);
-    const V tr = M::fma(M::c(2.f), sd, sxy);
+    const V tr = M::fma2p(2.f, sd, sxy);
     const V de0 = M::neg(M::add(sxy, sd));
     const V t12 = M::mul(tr, M::kc(1.f / 12.f, 1.0 / 12.0));
     const V dxy = M::sub(DX, DY), pxy = M::sub(DP, DM);
-    const V f1X = M::fma(dxy, M::c(0.25f), t12);
-    const V f1Y = M::fma(dxy, M::c(-0.25f), t12);
-    const V f1P = M::fma(pxy, M::c(0.25f), t12);
-    const V f1M = M::fma(pxy, M::c(-0.25f), t12);
+    V f1X, f1Y, f1P, f1M;
+    M::fma2p_pm(0.25f, dxy, t12, f1X, f1Y);
+    M::fma2p_pm(0.25f, pxy, t12, f1P, f1M);
     g[0] = M::add(g[0], M::fma(M::ck(k.d1t), tr, M::fma(M::ck(k.nkct), tr, M::mul(M::ck(k.kd), de0))));
     update_pair2_l<M, OP>(g[1], g[2], DX, DOX, f1X, k);
     update_pair2_l<M, OP>(g[3], g[4], DY, DOY, f1Y, k);

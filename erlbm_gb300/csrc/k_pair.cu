@@ -8,12 +8,18 @@ namespace erlbm {
 namespace {
 
 // One step of a periodic D2Q9 lattice: pull (mode 0) or the populations in place (mode 1, the first
-// step after they were set), then the compensated collision.  One node per thread.
+// step after they were set), then the compensated collision.  One node per thread.  Bound by the FP32 pipe: in 83 %
+// of the cycles a scheduler issues.  Two nodes a thread in packed FP32x2 arithmetic give the same time (1024^2: 43.97
+// and 43.68 us a step; packed operations run at the rate of single ones).  Launched after the step before it
+// programmatically (launch.cuh): 64^2 2.3 us a step.
+constexpr int PAIR_BLOCK = 128;
+
 template <int OP>
-__global__ void __launch_bounds__(256) k_step_pair(const float2 *__restrict__ src, float2 *__restrict__ dst, Geo g,
-                                                   int mode, pair32::CoefDS k)
+__global__ void __launch_bounds__(PAIR_BLOCK) k_step_pair(const float2 *__restrict__ src, float2 *__restrict__ dst, Geo g,
+                                                          int mode, pair32::CoefDS k)
 {
-    const long long node = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    after_previous();
+    const long long node = (long long)blockIdx.x * PAIR_BLOCK + threadIdx.x;
     if (node >= g.nbox) return;
     int x, y, z;
     node_xyz(g, node, x, y, z);
@@ -39,11 +45,11 @@ int launch_step_pair(int q, int op, const Geo &g, const Relax &R, int mode, cons
 {
     if (!step_pair_ok(q, op, g)) return -1;
     const pair32::CoefDS k = pair32::make_coef_ds(R);
-    const unsigned nb = blocks_for(g.nbox, 256);
+    const unsigned nb = blocks_for(g.nbox, PAIR_BLOCK);
     switch (op) {
-    case OP_BGK: k_step_pair<OP_BGK><<<nb, 256, 0, s>>>(src, dst, g, mode, k); break;
-    case OP_REG: k_step_pair<OP_REG><<<nb, 256, 0, s>>>(src, dst, g, mode, k); break;
-    default: k_step_pair<OP_EXTREG><<<nb, 256, 0, s>>>(src, dst, g, mode, k); break;
+    case OP_BGK: launch_step_kernel<k_step_pair<OP_BGK>, PAIR_BLOCK>(nb, s, src, dst, g, mode, k); break;
+    case OP_REG: launch_step_kernel<k_step_pair<OP_REG>, PAIR_BLOCK>(nb, s, src, dst, g, mode, k); break;
+    default: launch_step_kernel<k_step_pair<OP_EXTREG>, PAIR_BLOCK>(nb, s, src, dst, g, mode, k); break;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
