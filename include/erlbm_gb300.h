@@ -182,8 +182,9 @@ int erlbm_fp64_rate(double *ops_per_s);
  *   ERLBM_LAUNCH_STREAMING_STORES  evict-first stores (one-step kernel);
  *   ERLBM_LAUNCH_TWO_STEP          two consecutive steps per launch, the intermediate step kept on
  *                                  chip (nx % 128 == 0, ny even): half the HBM traffic per update;
- *   ERLBM_LAUNCH_THREE_STEP        three steps per launch (same conditions): a third of the traffic;
- *   ERLBM_LAUNCH_WIDE_STRIPS       with ERLBM_LAUNCH_THREE_STEP: 64-column warp strips in which a lane
+ *   ERLBM_LAUNCH_THREE_STEP        three steps per launch (same conditions): a third of the traffic, in
+ *                                  32-column warp strips, or 64-column ones where they are faster;
+ *   ERLBM_LAUNCH_WIDE_STRIPS       with ERLBM_LAUNCH_THREE_STEP: always 64-column warp strips, in which a lane
  *                                  holds two neighbouring columns (60 outputs per 64 columns instead
  *                                  of 28 per 32; ny >= 16 and 9 nx ny < 2^31, else one step per
  *                                  launch).
