@@ -146,7 +146,7 @@ __device__ __forceinline__ void moments9_fixed(const double f[9], int64_t F[9], 
     mx = round53(round53(round53(round53(mx + F[5]) - F[6]) + F[7]) - F[8]);
     my = round53(round53(round53(round53(my + F[5]) - F[6]) - F[7]) + F[8]);
     rho = fp64int::to_double(r);
-    const double inv = 1.0 / rho;
+    const double inv = fp64int::reciprocal(rho);
     ux = fp64int::to_double(mx) * inv;
     uy = fp64int::to_double(my) * inv;
 }

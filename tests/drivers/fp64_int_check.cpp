@@ -60,6 +60,16 @@ int main(int argc, char **argv)
             cases++;
         }
     }
+    // reciprocals, from first approximations off by up to 2^-20
+    for (long it = 0; it < n; it++) {
+        uint64_t M = rng() >> 12;
+        if (rng() % 3 == 0) M = rng() % 64;
+        if (rng() % 3 == 0) M = ~M & 0xfffffffffffffull;
+        const double r = from_bits(M | ((rng() % 8 ? 1023 - 3 + rng() % 8 : 513 + rng() % 1000) << 52));
+        double y = 0x1p32 / (1.0 + (double)M * 0x1p-52) * (1.0 + ((double)(rng() % 2001) - 1000.0) / 1000.0 * 0x1p-20);
+        cases++;
+        bad += bits(reciprocal_from(r, y >= 0x1p32 ? 0xffffffffu : (uint32_t)y)) != bits(1.0 / r);
+    }
     // quotients by a constant and by 3
     for (long it = 0; it < n; it++) {
         const double y = std::ldexp(1.0 + std::ldexp((double)(rng() >> 12), -52), (int)(rng() % 9) - 6);
