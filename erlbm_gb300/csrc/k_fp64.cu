@@ -133,39 +133,47 @@ int launch_box_field_fp64(int q, const Geo &g, const double *buf, int field, dou
 namespace {
 
 // Serial sum in index order: the reference's kinectic_energy loop (Other_functions.cpp:100-115), rounded
-// after every add as that loop is, by one warp.  One thread's chain of adds costs a load and an add
+// after every add as that loop is, by one block.  One thread's chain of adds costs a load and an add
 // latency per element (4096 elements: 170 us).  While the sum s stays in one binade [2^e, 2^(e+1)), with unit
 // u = 2^(e-52), adding x >= 0 rounds to s + u rint(x / u): what each element adds is an integer multiple of u
 // that does not depend on s, except at a tie.  So a chunk of SER_CHUNK elements is rounded in parallel and summed
-// exactly in 64-bit integers by a warp scan, up to the first element that takes s out of its binade, ties, or
+// exactly in 64-bit integers by a scan, up to the first element that takes s out of its binade, ties, or
 // is not a non-negative finite number; that element is added by a plain FP64 add, and the chunk goes on
-// behind it.  A sum of n similar terms leaves its binade log2(n) times.  A chunk with more than SER_STOPS
-// such elements (ties on equal inputs) is finished by a plain loop.  erlbm_kinetic_energy, launches and
-// read-back included: 4096 nodes 218 -> 68 us, 16384 784 -> 120, 65536 3040 -> 329.
+// behind it.  A sum of n similar terms leaves its binade log2(n) times and ties ln(n) times, which is what the
+// passes over a chunk are spent on.  A chunk with more than SER_STOPS such elements (ties on equal inputs) is
+// finished by a plain loop.  us of erlbm_kinetic_energy, launches and read-back (some 40) included, with one thread /
+// a warp / four warps / eight: 4096 nodes 214 / 66 / 55 / 60, 16384 781 / 129 / 80 / 79, 65536 3059 / 361 / 153 / 129.
+constexpr int SER_WARPS = 4;
+constexpr int SER_THREADS = 32 * SER_WARPS;
 constexpr int SER_PER_LANE = 8;
-constexpr int SER_CHUNK = 32 * SER_PER_LANE;
-constexpr int SER_STOPS = 24;
+constexpr int SER_CHUNK = SER_THREADS * SER_PER_LANE;
+constexpr int SER_STOPS = 34;
 
-__global__ void __launch_bounds__(32) k_sum_serial(const double *__restrict__ x, long long n, double *out)
+__global__ void __launch_bounds__(SER_THREADS) k_sum_serial(const double *__restrict__ x, long long n, double *out)
 {
     constexpr unsigned long long HIDDEN = 1ull << 52, MANT = HIDDEN - 1;
-    const int lane = threadIdx.x;
-    double s = 0.0;
+    // each pass uses the other set, so that a set is written again only after two barriers
+    __shared__ unsigned long long warp_sum[2][SER_WARPS], stop_sum[2][SER_WARPS];
+    __shared__ double stop_x[2][SER_WARPS];
+    __shared__ int stop_at[2][SER_WARPS];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double s = 0.0;  // the same in every thread
     double v[SER_PER_LANE], nx[SER_PER_LANE];
     auto load = [&](long long base, double w[SER_PER_LANE]) {
 #pragma unroll
         for (int j = 0; j < SER_PER_LANE; j++) {
-            const long long i = base + lane * SER_PER_LANE + j;
+            const long long i = base + tid * SER_PER_LANE + j;
             w[j] = i < n ? x[i] : 0.0;  // adding +0 changes nothing
         }
     };
     load(0, nx);
+    int set = 0;
     for (long long base = 0; base < n; base += SER_CHUNK) {
 #pragma unroll
         for (int j = 0; j < SER_PER_LANE; j++) v[j] = nx[j];
         load(base + SER_CHUNK, nx);
         int done = 0;  // elements of the chunk already in s
-        for (int stops = 0;; stops++) {
+        for (int stops = 0;; stops++, set ^= 1) {
             const unsigned long long sb = (unsigned long long)__double_as_longlong(s);
             const int se = (int)(sb >> 52);  // 0 for s = 0, > 2046 for a negative, infinite or NaN sum
             const bool in_binade = se >= 1 && se <= 2046;
@@ -180,7 +188,7 @@ __global__ void __launch_bounds__(32) k_sum_serial(const double *__restrict__ x,
             unsigned own = 0;
 #pragma unroll
             for (int j = 0; j < SER_PER_LANE; j++) {
-                const bool todo = lane * SER_PER_LANE + j >= done;
+                const bool todo = tid * SER_PER_LANE + j >= done;
                 const unsigned long long b = (unsigned long long)__double_as_longlong(v[j]);
                 const int xe = (int)(b >> 52);
                 const int sh = se - xe;
@@ -198,14 +206,26 @@ __global__ void __launch_bounds__(32) k_sum_serial(const double *__restrict__ x,
                 }
                 sum += q[j];
             }
+            // a thread whose elements alone leave the binade stops there, so what it hands on may be cut short:
+            // SER_THREADS times 4 HIDDEN fit 64 bits
+            sum = sum < 4 * HIDDEN ? sum : 4 * HIDDEN;
             unsigned long long incl = sum;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
                 if (lane >= o) incl += t;
             }
-            // the lane's first element that cannot be taken, with the sum before it
-            unsigned long long acc = S + (incl - sum), at = 0;
+            if (lane == 31) warp_sum[set][warp] = incl;
+            __syncthreads();
+            unsigned long long before = 0, total = S;
+#pragma unroll
+            for (int w = 0; w < SER_WARPS; w++) {
+                const unsigned long long t = warp_sum[set][w];
+                before += w < warp ? t : 0ull;
+                total += t;
+            }
+            // the thread's first element that cannot be taken, with the sum before it
+            unsigned long long acc = S + before + (incl - sum), at = 0;
             int stop = SER_PER_LANE;
 #pragma unroll
             for (int j = 0; j < SER_PER_LANE; j++) {
@@ -216,24 +236,32 @@ __global__ void __launch_bounds__(32) k_sum_serial(const double *__restrict__ x,
                 acc += q[j];
             }
             const unsigned who = __ballot_sync(0xffffffffu, stop < SER_PER_LANE);
-            if (who == 0) {
-                const unsigned long long total = __shfl_sync(0xffffffffu, acc, 31);
+            if (lane == (who ? __ffs(who) - 1 : 0)) {
+                double mine = 0.0;
+#pragma unroll
+                for (int j = 0; j < SER_PER_LANE; j++)
+                    if (j == stop) mine = v[j];
+                stop_at[set][warp] = who ? tid * SER_PER_LANE + stop : -1;
+                stop_sum[set][warp] = at;
+                stop_x[set][warp] = mine;
+            }
+            __syncthreads();
+            int first = SER_WARPS;
+#pragma unroll
+            for (int w = SER_WARPS - 1; w >= 0; w--)
+                if (stop_at[set][w] >= 0) first = w;
+            if (first == SER_WARPS) {
                 if (in_binade) s = __longlong_as_double((long long)((total & MANT) | ((unsigned long long)se << 52)));
+                set ^= 1;
                 break;
             }
-            const int first = __ffs(who) - 1;
-            const unsigned long long before = __shfl_sync(0xffffffffu, at, first);
-            double mine = 0.0;
-#pragma unroll
-            for (int j = 0; j < SER_PER_LANE; j++)
-                if (j == stop) mine = v[j];
-            const double xs = __shfl_sync(0xffffffffu, mine, first);
-            if (in_binade) s = __longlong_as_double((long long)((before & MANT) | ((unsigned long long)se << 52)));
-            s = s + xs;
-            done = first * SER_PER_LANE + __shfl_sync(0xffffffffu, stop, first) + 1;
+            if (in_binade)
+                s = __longlong_as_double((long long)((stop_sum[set][first] & MANT) | ((unsigned long long)se << 52)));
+            s = s + stop_x[set][first];
+            done = stop_at[set][first] + 1;
         }
     }
-    if (lane == 0) *out = s;
+    if (tid == 0) *out = s;
 }
 
 constexpr int RB = 256;   // threads per reduction block
@@ -325,7 +353,7 @@ __global__ void __launch_bounds__(RB) k_maxabs_final(const double *__restrict__ 
 int launch_sum(const double *x, long long n, long long serial_limit, double *scratch, double *out, cudaStream_t s)
 {
     if (n <= serial_limit) {
-        k_sum_serial<<<1, 32, 0, s>>>(x, n, out);
+        k_sum_serial<<<1, SER_THREADS, 0, s>>>(x, n, out);
     } else {
         k_sum_partial<<<RG, RB, 0, s>>>(x, n, scratch);
         k_sum_final<<<1, RB, 0, s>>>(scratch, out);
