@@ -512,6 +512,7 @@ int setup_planes_x3(erlbm_handle *h, const BCp &b)
     const int from[3] = {0, n[0], n[0] + n[1]};
     CK(cudaMemcpyAsync(at, from, sizeof(from), cudaMemcpyHostToDevice, h->stream));
     CKL(d2q9_fix_list(h->g, fix, h->d_x3_dist, at, h->d_x3_list, h->stream), "fix_list");
+    CK(cudaStreamSynchronize(h->stream));  // kernels that come in early read the list as read-only data
     h->x3_state = 1;
     return ERLBM_OK;
 }

@@ -19,21 +19,20 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-
 // Pull one direction plane for the four nodes x0..x0+3 of row y (periodic in x and y).
 template <int CX>
-__device__ __forceinline__ float4 pull4(const float *__restrict__ row, int x0, int xl, int xr, int lane)
+__device__ __forceinline__ float4 pull4(const float *row, int x0, int xl, int xr, int lane)
 {
-    const float4 a = __ldg(reinterpret_cast<const float4 *>(row + x0));
+    const float4 a = *reinterpret_cast<const float4 *>(row + x0);
     if (CX == 0) return a;
     if (CX == 1) {  // values at x0-1 .. x0+2
-        const float e = (lane == 0) ? __ldg(row + xl) : 0.f;
+        const float e = (lane == 0) ? row[xl] : 0.f;
         float p = __shfl_up_sync(FULL, a.w, 1);
         if (lane == 0) p = e;
         return make_float4(p, a.x, a.y, a.z);
     }
     // CX == -1: values at x0+1 .. x0+4
-    const float e = (lane == 31) ? __ldg(row + xr) : 0.f;
+    const float e = (lane == 31) ? row[xr] : 0.f;
     float n = __shfl_down_sync(FULL, a.x, 1);
     if (lane == 31) n = e;
     return make_float4(a.y, a.z, a.w, n);
@@ -66,7 +65,7 @@ __device__ __forceinline__ void store4(float *p, const float4 &v)
 }
 
 template <int OP, int BLOCK, bool STREAMING>
-__global__ void __launch_bounds__(BLOCK) k_periodic_d2q9(const float *__restrict__ src, float *__restrict__ dst, int nx,
+__global__ void __launch_bounds__(BLOCK) k_periodic_d2q9(const float *src, float *__restrict__ dst, int nx,
                                                           int ny, long long plane, shifted::Coef k)
 {
     after_previous();
@@ -153,7 +152,7 @@ constexpr int XS_W = 30;
 constexpr unsigned XS_FULL = 0xffffffffu;
 
 template <int OP>
-__global__ void __launch_bounds__(128) k_periodic_d2q9_x2s(const float *__restrict__ src, float *__restrict__ dst,
+__global__ void __launch_bounds__(128) k_periodic_d2q9_x2s(const float *src, float *__restrict__ dst,
                                                           int nx, int ny, long long plane, int hc, int strips,
                                                           int n_warps, shifted::Coef k)
 {
@@ -179,11 +178,11 @@ __global__ void __launch_bounds__(128) k_periodic_d2q9_x2s(const float *__restri
         r = r < 0 ? r + ny : (r >= ny ? r - ny : r);
         const float *p = src + (long long)r * nx;
 #pragma unroll
-        for (int i = 0; i < 9; i++) v[i] = __ldg(p + c + i * plane);
+        for (int i = 0; i < 9; i++) v[i] = p[c + i * plane];
         if (halo) {
-            h[0] = __ldg(p + h0);
-            h[1] = __ldg(p + h1);
-            h[2] = __ldg(p + h2);
+            h[0] = p[h0];
+            h[1] = p[h1];
+            h[2] = p[h2];
         }
     };
     // a[i] = P(column - cx_i) of the loaded row
@@ -311,7 +310,7 @@ constexpr int X3_W = 28;
 constexpr int X3_SKIP = 2;
 
 template <int OP, bool SKIP>
-__global__ void __launch_bounds__(128, 4) k_periodic_d2q9_x3s(const float *__restrict__ src, float *__restrict__ dst,
+__global__ void __launch_bounds__(128, 4) k_periodic_d2q9_x3s(const float *src, float *__restrict__ dst,
                                                           int nx, int ny, long long plane, int hc, int strips,
                                                           int n_warps, const uint8_t *__restrict__ dist,
                                                           shifted::Coef k)
@@ -335,11 +334,11 @@ __global__ void __launch_bounds__(128, 4) k_periodic_d2q9_x3s(const float *__res
         r = r < 0 ? r + ny : (r >= ny ? r - ny : r);
         const float *p = src + (long long)r * nx;
 #pragma unroll
-        for (int i = 0; i < 9; i++) v[i] = __ldg(p + c + i * plane);
+        for (int i = 0; i < 9; i++) v[i] = p[c + i * plane];
         if (halo) {
-            h[0] = __ldg(p + h0);
-            h[1] = __ldg(p + h1);
-            h[2] = __ldg(p + h2);
+            h[0] = p[h0];
+            h[1] = p[h1];
+            h[2] = p[h2];
         }
     };
     auto align = [&](const float v[9], const float h[3], float a[9]) {
@@ -535,7 +534,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 template <int OP, int MINB, bool SKIP>
-__global__ void __launch_bounds__(128, MINB) k_periodic_d2q9_x3a(const float *__restrict__ src, float *__restrict__ dst,
+__global__ void __launch_bounds__(128, MINB) k_periodic_d2q9_x3a(const float *src, float *__restrict__ dst,
                                                                 int nx, int ny, int plane, int hc, int strips,
                                                                 int n_warps, const uint8_t *__restrict__ dist,
                                                                 shifted::Coef k)
@@ -894,7 +893,7 @@ __device__ __forceinline__ unsigned fdiv(unsigned n, const FastDiv &f)
 // (4470 -> 6350 GB/s), 192^3: 226.8 -> 158.2 us (6800 GB/s, the measured copy rate), 64^3 (in L2): 10.3 ->
 // 8.3 us; 32^3 and below stay at the launch rate.
 template <int OP>
-__global__ void __launch_bounds__(128, 6) k_periodic_d3q19(const float *__restrict__ src, float *__restrict__ dst,
+__global__ void __launch_bounds__(128, 6) k_periodic_d3q19(const float *src, float *__restrict__ dst,
                                                             unsigned nx, unsigned ny, unsigned nz, unsigned nbox,
                                                             size_t plane, FastDiv fx, FastDiv fy, shifted::Coef k)
 {
@@ -913,7 +912,7 @@ __global__ void __launch_bounds__(128, 6) k_periodic_d3q19(const float *__restri
         const int cx = Lat<19>::cx(i), cy = Lat<19>::cy(i), cz = Lat<19>::cz(i);
         const unsigned s = node + (cx == 1 ? xm : (cx == -1 ? xp : 0u)) + (cy == 1 ? ym : (cy == -1 ? yp : 0u)) +
                            (cz == 1 ? zm : (cz == -1 ? zp : 0u));
-        f[i] = __ldg(src + (size_t)i * plane + s);
+        f[i] = src[(size_t)i * plane + s];
     }
     shifted::collide<19, OP>(f, k);
 #pragma unroll
@@ -963,7 +962,7 @@ namespace {
 // fused update but never read (the pull of a fluid node that faces a solid takes its own opposite
 // population), so what it holds does not matter.  Both updates give the generic kernel's bits.
 template <int OP>
-__global__ void __launch_bounds__(256) k_d2q9_hybrid(const float *__restrict__ src, float *__restrict__ dst, Geo g,
+__global__ void __launch_bounds__(256) k_d2q9_hybrid(const float *src, float *__restrict__ dst, Geo g,
                                                      BCp bc, CollParams prm, const uint8_t *__restrict__ segflag,
                                                      const uint8_t *__restrict__ nodeflag,
                                                      const int *__restrict__ fix, int n_fix, int n_fix_blocks)
@@ -1192,7 +1191,7 @@ __global__ void __launch_bounds__(256) k_fix_list(Geo g, const uint8_t *__restri
 // the plane nodes have warps of their own: among the others, in row order, one of them would hold up a
 // warp per row (9.2 -> 6.8 us per launch on the 4096 x 1024 channel).
 template <int OP>
-__global__ void __launch_bounds__(64) k_listed_step(const float *__restrict__ src, float *__restrict__ dst, Geo g,
+__global__ void __launch_bounds__(64) k_listed_step(const float *src, float *__restrict__ dst, Geo g,
                                                     BCp bc, shifted::Coef k, const int *__restrict__ list, int n_list,
                                                     int n_planes)
 {

@@ -18,7 +18,7 @@ namespace {
 constexpr int QUAD_BLOCK = 64;
 
 template <int Q, int OP>
-__global__ void __launch_bounds__(QUAD_BLOCK) k_step_quad(const double *__restrict__ src, double *__restrict__ dst, Geo g,
+__global__ void __launch_bounds__(QUAD_BLOCK) k_step_quad(const double *src, double *__restrict__ dst, Geo g,
                                                           BCp bc, Relax R, StepArgs a)
 {
     after_previous();

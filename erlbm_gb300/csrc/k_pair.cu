@@ -15,7 +15,7 @@ namespace {
 constexpr int PAIR_BLOCK = 128;
 
 template <int OP>
-__global__ void __launch_bounds__(PAIR_BLOCK) k_step_pair(const float2 *__restrict__ src, float2 *__restrict__ dst, Geo g,
+__global__ void __launch_bounds__(PAIR_BLOCK) k_step_pair(const float2 *src, float2 *__restrict__ dst, Geo g,
                                                           int mode, pair32::CoefDS k)
 {
     after_previous();

@@ -260,7 +260,7 @@ __device__ __forceinline__ T ldx(const T *p)
 // direction i is node (x - c_x, y - c_y, z - c_z) with periodic wrap: its index is the node's plus
 // one offset per axis, set once for the node's position.
 template <class P, int Q, bool COH = false>
-__device__ __forceinline__ void gather(const typename P::T *__restrict__ src, const Geo &g, int mode, int x, int y,
+__device__ __forceinline__ void gather(const typename P::T *src, const Geo &g, int mode, int x, int y,
                                        int z, long long node, typename P::T *f)
 {
     if (mode == 1) {
@@ -327,7 +327,7 @@ __device__ __forceinline__ void apply_inlet(typename P::T *f, const Geo &g, cons
 
 // Populations of fluid node (x, y, z) after this step's inlet and outlet planes.
 template <class P, int Q, bool COH = false>
-__device__ void state_after_x_planes(const typename P::T *__restrict__ src, const Geo &g, const BCp &bc, int mode,
+__device__ void state_after_x_planes(const typename P::T *src, const Geo &g, const BCp &bc, int mode,
                                      int x, int y, int z, long long node, typename P::T *f)
 {
     using T = typename P::T;
@@ -373,7 +373,7 @@ __device__ void state_after_x_planes(const typename P::T *__restrict__ src, cons
 
 // Post-boundary populations of fluid node (x, y, z): the x planes, then OpenBoundaryD2Q9_y.
 template <class P, int Q, bool COH = false>
-__device__ void state_after_planes(const typename P::T *__restrict__ src, const Geo &g, const BCp &bc, int mode, int x,
+__device__ void state_after_planes(const typename P::T *src, const Geo &g, const BCp &bc, int mode, int x,
                                    int y, int z, long long node, typename P::T *f)
 {
     state_after_x_planes<P, Q, COH>(src, g, bc, mode, x, y, z, node, f);
@@ -405,7 +405,7 @@ __device__ void state_after_planes(const typename P::T *__restrict__ src, const 
 // of a density the check has seen; a node whose density is certainly below it returns 0.  The body
 // of k_step, shared with the resident team loop so that both give the same bits.
 template <class P, int Q, int OP, bool COH = false>
-__device__ __forceinline__ void step_node(const typename P::T *__restrict__ src, typename P::T *__restrict__ dst,
+__device__ __forceinline__ void step_node(const typename P::T *src, typename P::T *__restrict__ dst,
                                           const Geo &g, const BCp &bc, const CollParams &prm, int mode,
                                           int check_density, double density_limit, long long node,
                                           unsigned long long &rho_bits, int &flag, uint32_t known = 0)
@@ -447,7 +447,7 @@ __device__ __forceinline__ void report_density(RunStatus *status, int step_index
 }
 
 template <class P, int Q, int OP>
-__global__ void __launch_bounds__(256) k_step(const typename P::T *__restrict__ src, typename P::T *__restrict__ dst,
+__global__ void __launch_bounds__(256) k_step(const typename P::T *src, typename P::T *__restrict__ dst,
                                               Geo g, BCp bc, CollParams prm, StepArgs a)
 {
     after_previous();

@@ -17,6 +17,10 @@ namespace erlbm {
 // until the kernel before it in the stream has finished and its writes are visible, then lets the next one be
 // launched (to wait in its turn).  The order matters: a successor that was brought in while this kernel still waits
 // could keep lines in its L1 of the buffer that the kernel before this one reads and this one writes.
+// What an earlier kernel of the stream writes (the populations) is read by ordinary loads, from pointers without
+// __restrict__: the read-only path (__ldg, const __restrict__) is for data that nobody writes while the kernel is
+// resident, which for a kernel that comes in early includes the time before this wait, and the compiler may move such
+// loads above it.
 __device__ __forceinline__ void after_previous()
 {
     asm volatile("griddepcontrol.wait;" ::: "memory");
