@@ -251,11 +251,24 @@ struct BatchSmem {
 // except that the nodes of the boundary planes are packed together.  Those run the inlet and outlet closures
 // (with FP64 operations in the FP32 path); packed, they do not put that work on every warp of the CTA in every
 // step.  Solid nodes get no thread.
-// FP32: both planes first, in one warp.  FP64 (apart): a warp's FP64 instructions hold its scheduler's pipe however
+// FP32: both planes first, in one warp.  FP64 (APART): a warp's FP64 instructions hold its scheduler's pipe however
 // few of its lanes take part, so each plane gets a warp of its own, and the CTAs of the grid's second half, which
 // share their SMs with those of the first, the next two, so that four schedulers take the four planes' closures.
-__device__ inline void make_order(const BatchGeo &g, short *order, int *n_fluid, const uint8_t *solid, bool apart)
+template <bool APART>
+__device__ inline void make_order(const BatchGeo &g, short *order, int *n_fluid, const uint8_t *solid)
 {
+    if constexpr (!APART) {
+        int k = 0;
+        for (int pass = 0; pass < 2; pass++)
+            for (int n = 0; n < g.nb; n++) {
+                if (solid[n]) continue;
+                const int x = n % g.nx;
+                const bool plane = x == g.inlet_x || x == g.outlet_x;
+                if (plane == (pass == 0)) order[k++] = (short)n;
+            }
+        *n_fluid = k;
+        return;
+    }
     int n_all = 0, n_in = 0, n_out = 0;
     for (int n = 0; n < g.nb; n++) {
         if (solid[n]) continue;
@@ -265,7 +278,7 @@ __device__ inline void make_order(const BatchGeo &g, short *order, int *n_fluid,
         n_out += x == g.outlet_x && x != g.inlet_x;
     }
     int in = 0, out = n_in;  // first slots of the planes
-    if (apart && n_in <= 32 && n_out <= 32 && n_all >= 128) {
+    if (n_in <= 32 && n_out <= 32 && n_all >= 128) {
         in = 2 * blockIdx.x >= gridDim.x ? 64 : 0;
         out = in + 32;
         if (out + n_out > n_all) {
@@ -278,9 +291,7 @@ __device__ inline void make_order(const BatchGeo &g, short *order, int *n_fluid,
     for (int n = 0; n < g.nb; n++) {
         if (solid[n]) continue;
         const int x = n % g.nx;
-        if (!apart && (x == g.inlet_x || x == g.outlet_x)) {
-            order[a++] = (short)n;  // node order over both planes
-        } else if (x == g.inlet_x) {
+        if (x == g.inlet_x) {
             order[a++] = (short)n;
         } else if (x == g.outlet_x) {
             order[b++] = (short)n;
@@ -335,13 +346,17 @@ __device__ BatchResult batch_one_run(const BatchGeo &g, const BatchRun &r, const
     if (tid == 0) *reinterpret_cast<ZH *>(sm.zh) = P::zou_he_prep_run(r.u0);
     if (tid == 0) *sm.known = 0;
 
-    // directions that come back from a solid neighbour, a bit each: found once a run, where a lookup in every step
-    // was a byte from shared memory per direction
+    // Directions that come back from a solid neighbour, a bit each, found once a run, where a look-up in every step is
+    // a byte from shared memory per direction: FP64, and FP32 with a node a thread (the resident slot loop, 800 obstacle
+    // runs of 2000 steps 93 -> 28.7 ms).  FP32 CTAs of several nodes a thread (k_batch) have the registers and issue
+    // slots for the look-up, and run slower with a mask and a select per direction: obstacle map of 2000 runs of 1000
+    // steps 12.6 -> 14.0 ms, periodic Taylor-Green runs on 20^2 nodes 4.7 -> 5.8 ms.
+    constexpr bool MASK = sizeof(T) == 8 || NPT == 1;
     uint32_t bounce[NPT];
 #pragma unroll
     for (int s = 0; s < NPT; s++) {
         bounce[s] = 0;
-        if (!any_solid || !fluid[s]) continue;
+        if (!MASK || !any_solid || !fluid[s]) continue;
         int x = nx_[s];
         if (x == g.outlet_x) x += (g.outlet_x < g.nx / 2) ? 1 : -1;  // the outlet copies its inner neighbour
 #pragma unroll
@@ -407,7 +422,10 @@ __device__ BatchResult batch_one_run(const BatchGeo &g, const BatchRun &r, const
                     const int xs = wrap1(x - Lat<Q>::cx(i), g.nx);
                     const int ys = wrap1(y - Lat<Q>::cy(i), g.ny);
                     const int src = xs + g.nx * ys;
-                    f[s][i] = cur[bounce[s] >> i & 1u ? Lat<Q>::opp(i) * NB + me : i * NB + src];
+                    if constexpr (MASK)
+                        f[s][i] = cur[bounce[s] >> i & 1u ? Lat<Q>::opp(i) * NB + me : i * NB + src];
+                    else
+                        f[s][i] = (any_solid && solid[src]) ? cur[Lat<Q>::opp(i) * NB + me] : cur[i * NB + src];
                 }
             }
         } else if (g.outlet_x >= 0) {
@@ -555,7 +573,7 @@ __global__ void __launch_bounds__(MAXT, BatchBounds<NPT, sizeof(typename P::T)>:
     const int tid = threadIdx.x;
     for (int k = tid; k < g.nb; k += blockDim.x) sm.solid[k] = g.solid ? g.solid[k] : 0;
     __syncthreads();
-    if (tid == 0) make_order(g, sm.order, sm.n_fluid, sm.solid, sizeof(typename P::T) == 8 && NPT == 1);
+    if (tid == 0) make_order<sizeof(typename P::T) == 8 && NPT == 1>(g, sm.order, sm.n_fluid, sm.solid);
     for (;;) {
         __syncthreads();
         if (tid == 0) s_run = atomicAdd(counter, 1);
@@ -661,7 +679,7 @@ __global__ void __launch_bounds__(BatchBounds<NPT, sizeof(typename P::T)>::MAXT,
         for (int k = tid; k < g.nb && k < max_nb; k += blockDim.x) sm.solid[k] = g.solid ? g.solid[k] : 0;
         __syncthreads();
         if (tid == 0 && g.nb <= max_nb)
-            make_order(g, sm.order, sm.n_fluid, sm.solid, sizeof(typename P::T) == 8 && NPT == 1);
+            make_order<sizeof(typename P::T) == 8 && NPT == 1>(g, sm.order, sm.n_fluid, sm.solid);
         __syncthreads();
         BatchResult o;
         if (g.nb > max_nb || g.nb > NPT * (int)blockDim.x) {
