@@ -124,8 +124,9 @@ struct PrecExact64 {
     __device__ static __forceinline__ double to_f(T v, int) { return v; }
 };
 
-// The exact path for MRT lattices and lattices past four lanes a node (k_fp64.cu) of fewer warps than hide the latency of the fixed-point sums: the same bits with
-// more FP64 operations and fewer dependent integer ones.
+// The exact path where a scheduler has fewer warps than hide the latency of the fixed-point sums: lattices below
+// FIXED_MIN_NODES that do not take four lanes a node (k_fp64.cu), the resident team loop of one CTA an SM
+// (k_team64.cu).  The same bits with more FP64 operations and fewer dependent integer ones.
 struct PrecExact64Small : PrecExact64 {
     template <int Q, int OP>
     __device__ static __forceinline__ void collide(T *f, const CollParams &p)
