@@ -95,3 +95,29 @@ def test_fp64_collision_of_larger_lattices(q, shape, kind):
         want = ref.get(1)
         fine = np.isfinite(want)
         assert np.array_equal(np.isfinite(got), fine) and np.array_equal(got[fine], want[fine])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("q,nx,ny", [(9, 16, 16), (9, 24, 23), (9, 33, 31), (19, 12, 10), (19, 16, 17), (19, 21, 20)])
+@pytest.mark.parametrize("kind", ["mach", "fast", "dense", "noise"])
+def test_batched_fp64_runs_of_states_mixed_among_the_lanes(q, nx, ny, kind):
+    """Batched runs (one, two and four nodes a thread) whose warps have lanes in and out of the ranges of the integer
+    forms: the greatest density of four steps, bit for bit."""
+    import erlbm_gb300 as E
+    n, limit = nx * ny, 1e6
+    runs, blocks, want = [], [], []
+    for k, op in enumerate((3, 4, 1)):
+        f = states(q, n, kind, np.random.default_rng(10 * n + k))
+        tnh = 1.0 if op == 3 else 0.65
+        ref = O.Lattice(q, nx, ny, 1, None, 0.6, tnh, op)
+        ref.set(f)
+        most = 0.0
+        for _ in range(4):
+            ref.step(1)
+            most = max(most, ref.max_abs_density(1)[0])
+        runs.append(dict(op=op, tau=0.6, tau_nh=tnh, u0=0.0, n_steps=4, aos_offset=k * f.size))
+        blocks.append(f)
+        want.append(most / limit)
+    got = E.batch_run(q, nx, ny, runs, precision=E.FP64, init=E.INIT_AOS, aos=np.concatenate(blocks),
+                      density_check=True, density_limit=limit)
+    assert [g["margin"] for g in got] == want
