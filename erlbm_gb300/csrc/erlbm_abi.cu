@@ -572,7 +572,18 @@ int bc_graph_steps(erlbm_handle *h, const BCp &b, bool by_three)
 // gains 19 us on 4096 x 1024 nodes, 2.6 us on 1000 x 250.
 int x3_setup_steps(const erlbm_handle *h) { return h->g.nbox >= 1000000 ? 48 : 192; }
 
-// n_steps steps without checks, by graph blocks and multi-step launches where they apply.
+// Whether the caller is recording the handle's stream into a graph of its own (erlbm_set_stream).
+bool being_recorded(const erlbm_handle *h)
+{
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(h->stream, &st) != cudaSuccess) cudaGetLastError();
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// n_steps steps without checks, by graph blocks and multi-step launches where they apply.  A call that is being
+// recorded gives plain launches only: a graph can be neither built nor launched into a recording, the set-up of three
+// steps with planes waits for the stream, and its lists, which a later set-up frees, must not get into a graph that the
+// caller keeps.
 int advance(erlbm_handle *h, int n_steps, const BCp &b)
 {
     int rc;
@@ -581,8 +592,9 @@ int advance(erlbm_handle *h, int n_steps, const BCp &b)
     PeriodicPlan p;
     if (plain) p = periodic_plan(h);
     const bool hybrid = fp32_2d && !plain && d2q9_hybrid_ok(h->g);
+    const bool recorded = fp32_2d && being_recorded(h);
     bool by_three = false;
-    if (fp32_2d && !plain && d2q9_planes_x3_ok(h->g)) {
+    if (fp32_2d && !plain && !recorded && d2q9_planes_x3_ok(h->g)) {
         auto current = [&] {
             return h->x3_state != 0 && h->x3_planes[0] == b.inlet_x && h->x3_planes[1] == b.outlet_x &&
                    h->x3_planes[2] == b.open_y;
@@ -594,7 +606,7 @@ int advance(erlbm_handle *h, int n_steps, const BCp &b)
     }
     for (int s = 0; s < n_steps;) {
         const int left = n_steps - s;
-        if ((hybrid || by_three) && h->kind == 1 && left >= bc_graph_steps_of(by_three)) {
+        if (!recorded && (hybrid || by_three) && h->kind == 1 && left >= bc_graph_steps_of(by_three)) {
             if ((rc = bc_graph_steps(h, b, by_three))) return rc;
             s += bc_graph_steps_of(by_three);
             continue;
@@ -607,7 +619,7 @@ int advance(erlbm_handle *h, int n_steps, const BCp &b)
             continue;
         }
         if (plain && h->kind == 1 && (p.per_launch > 1 || p.fused1)) {
-            if (left >= graph_steps_of(p.per_launch)) {
+            if (!recorded && left >= graph_steps_of(p.per_launch)) {
                 if ((rc = graph_steps(h, p))) return rc;
                 s += graph_steps_of(p.per_launch);
                 continue;
