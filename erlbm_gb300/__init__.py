@@ -123,6 +123,12 @@ class Lattice:
                  (8 if wide_strips else 0))
         check(lib().erlbm_set_launch(self._h, int(block_threads), flags), "erlbm_set_launch")
 
+    def launch_form(self):
+        """(steps per launch, 64-column strips) of the last step or run call: the most that one launch took."""
+        n, w = C.c_int(), C.c_int()
+        check(lib().erlbm_launch_form(self._h, C.byref(n), C.byref(w)), "erlbm_launch_form")
+        return n.value, bool(w.value)
+
     def kinetic_energy(self, stage: int = STAGE_POST_STREAM) -> float:
         e = C.c_double()
         check(lib().erlbm_kinetic_energy(self._h, stage, C.byref(e)), "erlbm_kinetic_energy")

@@ -102,12 +102,17 @@ struct erlbm_handle {
     BCp bc_graph_bc{};
     bool bc_graph_by_three = false;
     // three steps per launch with solids or planes (launch_d2q9_planes_x3), set up for the planes x3_planes
-    // by the first call that has steps enough; x3_state: 0 not tried, 1 ready, -1 not for these planes
+    // once calls in a row have asked for steps enough with them (x3_seen, x3_asked); x3_state: 0 not set up,
+    // 1 ready, -1 not for these planes
     int x3_state = 0, x3_planes[3] = {-1, -1, -1}, x3_listed[3] = {0, 0, 0};
-    uint8_t *d_x3_dist = nullptr;
+    int x3_seen[3] = {-1, -1, -1};
+    long long x3_asked = 0;
+    uint8_t *d_x3_dist = nullptr;       // node distances, then the nodes' kinds (d2q9_fix_distance)
     int *d_x3_list = nullptr;
     float *d_x3_mid = nullptr;
     cudaStream_t capture_stream = nullptr;
+    int form_steps = 0;                 // erlbm_launch_form
+    bool form_wide = false;
     size_t elem() const { return prec == ERLBM_FP32_SHIFTED ? sizeof(float) : 8; }  // FP64 or a float pair
 };
 
@@ -154,6 +159,17 @@ void drop_graphs(erlbm_handle *h)
     drop_bc_graphs(h);
 }
 
+void drop_planes_x3(erlbm_handle *h)
+{
+    cudaFree(h->d_x3_dist);
+    cudaFree(h->d_x3_list);
+    cudaFree(h->d_x3_mid);
+    h->d_x3_dist = nullptr;
+    h->d_x3_list = nullptr;
+    h->d_x3_mid = nullptr;
+    h->x3_state = 0;
+}
+
 void free_handle(erlbm_handle *h)
 {
     if (!h) return;
@@ -161,9 +177,7 @@ void free_handle(erlbm_handle *h)
     cudaFree(h->d_segflag);
     cudaFree(h->d_nodeflag);
     cudaFree(h->d_fix);
-    cudaFree(h->d_x3_dist);
-    cudaFree(h->d_x3_list);
-    cudaFree(h->d_x3_mid);
+    drop_planes_x3(h);
     cudaFree(h->d_profile);
     cudaFree(h->d_nof);
     cudaFree(h->d_buf[0]);
@@ -339,6 +353,14 @@ int validate_bc(erlbm_handle *h, const erlbm_bc *bc, BCp *out)
     return ERLBM_OK;
 }
 
+// Notes a launch of `steps` steps for erlbm_launch_form.
+void took(erlbm_handle *h, int steps, bool wide)
+{
+    if (steps < h->form_steps) return;
+    h->form_steps = steps;
+    h->form_wide = wide;
+}
+
 // Enqueue one step.  status/check_density are used by erlbm_run.
 int enqueue_step(erlbm_handle *h, const BCp &bc, int check_density, double density_limit, bool stop_on_flag)
 {
@@ -377,6 +399,7 @@ int enqueue_step(erlbm_handle *h, const BCp &bc, int check_density, double densi
     } else {
         CKL(launch_step_fp32(h->q, h->op, h->g, bc, h->R, a, (const float *)src, (float *)dst, h->stream), "step");
     }
+    took(h, 1, false);
     h->cur ^= 1;
     h->kind = 1;
     h->steps_done++;
@@ -478,24 +501,26 @@ bool same_planes(const BCp &a, const BCp &b)
 }
 
 // Sets up three steps per launch for the planes b: node distances, the list of nodes that take the generic
-// update, the scratch buffer of the middle step.  Left to single steps (x3_state = -1) when more than a
-// quarter of the nodes would be listed or device memory is short.
+// update, the scratch buffer of the middle step (a third population buffer and two bytes per node, kept until the
+// handle goes).  Left to single steps, with nothing kept, when more than a quarter of the nodes would be listed
+// (x3_state = -1) or device memory is short (0: tried again after as many steps).
 int setup_planes_x3(erlbm_handle *h, const BCp &b)
 {
     const int planes[3] = {b.inlet_x, b.outlet_x, b.open_y};
     CK(cudaStreamSynchronize(h->stream));  // steps in flight may read the lists of other planes
     drop_bc_graphs(h);
     memcpy(h->x3_planes, planes, sizeof(planes));
-    h->x3_state = -1;
+    h->x3_state = 0;
+    h->x3_asked = 0;
     cudaFree(h->d_x3_list);
     h->d_x3_list = nullptr;
-    const size_t pop_bytes = (size_t)h->q * h->g.plane * sizeof(float);
-    if ((!h->d_x3_dist && cudaMalloc(&h->d_x3_dist, h->g.nbox) != cudaSuccess) ||
-        (!h->d_x3_mid && cudaMalloc(&h->d_x3_mid, pop_bytes) != cudaSuccess)) {
+    auto no_memory = [h] {
         cudaGetLastError();
+        drop_planes_x3(h);
         return ERLBM_OK;
-    }
-    uint8_t *fix = (uint8_t *)h->d_x3_mid;  // free until the first step
+    };
+    if (!h->d_x3_dist && cudaMalloc(&h->d_x3_dist, 2 * h->g.nbox) != cudaSuccess) return no_memory();
+    uint8_t *fix = h->d_x3_dist + h->g.nbox;
     int *at = (int *)h->d_out, *n = h->x3_listed;
     CK(cudaMemsetAsync(at, 0, 3 * sizeof(int), h->stream));
     CKL(d2q9_fix_distance(h->g, b, fix, h->d_x3_dist, h->stream), "fix_distance");
@@ -503,11 +528,18 @@ int setup_planes_x3(erlbm_handle *h, const BCp &b)
     CK(cudaMemcpyAsync(n, at, sizeof(h->x3_listed), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     const long long all = (long long)n[0] + n[1] + n[2];
-    if (all > h->g.nbox / 4) return ERLBM_OK;
-    if (cudaMalloc(&h->d_x3_list, (all > 0 ? all : 1) * sizeof(int)) != cudaSuccess) {
-        cudaGetLastError();
-        h->d_x3_list = nullptr;
+    if (all > h->g.nbox / 4) {
+        drop_planes_x3(h);
+        h->x3_state = -1;
         return ERLBM_OK;
+    }
+    if (cudaMalloc(&h->d_x3_list, (all > 0 ? all : 1) * sizeof(int)) != cudaSuccess) {
+        h->d_x3_list = nullptr;
+        return no_memory();
+    }
+    if (!h->d_x3_mid && cudaMalloc(&h->d_x3_mid, (size_t)h->q * h->g.plane * sizeof(float)) != cudaSuccess) {
+        h->d_x3_mid = nullptr;
+        return no_memory();
     }
     const int from[3] = {0, n[0], n[0] + n[1]};
     CK(cudaMemcpyAsync(at, from, sizeof(from), cudaMemcpyHostToDevice, h->stream));
@@ -568,9 +600,39 @@ int bc_graph_steps(erlbm_handle *h, const BCp &b, bool by_three)
     return ERLBM_OK;
 }
 
-// Steps from which the set-up of three steps per launch with planes pays: it costs some 0.4 to 0.7 ms, and a step
-// gains 19 us on 4096 x 1024 nodes, 2.6 us on 1000 x 250.
-int x3_setup_steps(const erlbm_handle *h) { return h->g.nbox >= 1000000 ? 48 : 192; }
+// Steps after which three steps per launch with planes have paid for their set-up and the graphs that follow, some 0.45
+// to 0.8 ms.  What a step gains depends on the box: us per single step (k_d2q9_hybrid where nx % 128 == 0, the
+// generic kernel elsewhere), by threes, and the steps that pay: generic 1500 x 375 12.0 / 9.7, 180; 1600 x 400 12.3 / 10.4,
+// 225; 1000 x 700 14.4 / 10.2, 104; 2000 x 500 18.2 / 12.3, 86; 2800 x 700 42.7 / 17.2, 25; 3600 x 900 68.3 / 23.8, 16;
+// hybrid 1536 x 1024 17.5 / 15.8, 240; 2560 x 640 18.0 / 15.8, 180; 2816 x 704 23.2 / 17.6, 84; 2048 x 1536 36.9 / 24.6, 43;
+// 4096 x 1024 46.8 / 28.3, 28.  Below half a million and one and a half million nodes the threes gain nothing
+// (d2q9_planes_x3_ok).
+long long x3_setup_steps(const erlbm_handle *h)
+{
+    return 80000000 / (h->g.nbox - (d2q9_hybrid_ok(h->g) ? 1400000 : 400000)) + 16;
+}
+
+// Whether steps with the planes b go by threes, n_steps of them asked for now; sets them up when due.
+int planes_by_three(erlbm_handle *h, const BCp &b, int n_steps, bool *yes)
+{
+    const int planes[3] = {b.inlet_x, b.outlet_x, b.open_y};
+    *yes = false;
+    if (n_steps < 3 || !d2q9_planes_x3_ok(h->g)) return ERLBM_OK;
+    auto current = [&] { return h->x3_state != 0 && memcmp(h->x3_planes, planes, sizeof(planes)) == 0; };
+    if (memcmp(h->x3_seen, planes, sizeof(planes)) != 0) {
+        memcpy(h->x3_seen, planes, sizeof(planes));
+        h->x3_asked = 0;
+    }
+    if (!current()) {
+        h->x3_asked += n_steps;
+        if (h->x3_asked >= x3_setup_steps(h)) {
+            const int rc = setup_planes_x3(h, b);
+            if (rc) return rc;
+        }
+    }
+    *yes = h->x3_state == 1 && current();
+    return ERLBM_OK;
+}
 
 // Whether the caller is recording the handle's stream into a graph of its own (erlbm_set_stream).
 bool being_recorded(const erlbm_handle *h)
@@ -594,25 +656,20 @@ int advance(erlbm_handle *h, int n_steps, const BCp &b)
     const bool hybrid = fp32_2d && !plain && d2q9_hybrid_ok(h->g);
     const bool recorded = fp32_2d && being_recorded(h);
     bool by_three = false;
-    if (fp32_2d && !plain && !recorded && d2q9_planes_x3_ok(h->g)) {
-        auto current = [&] {
-            return h->x3_state != 0 && h->x3_planes[0] == b.inlet_x && h->x3_planes[1] == b.outlet_x &&
-                   h->x3_planes[2] == b.open_y;
-        };
-        // a call with few steps does not pay for the set-up
-        if (n_steps >= x3_setup_steps(h) && !current())
-            if ((rc = setup_planes_x3(h, b))) return rc;
-        by_three = h->x3_state == 1 && current();
-    }
+    if (fp32_2d && !plain && !recorded)
+        if ((rc = planes_by_three(h, b, n_steps, &by_three))) return rc;
+    const bool planes_wide = by_three && periodic_d2q9_prefers_wide(h->g);
     for (int s = 0; s < n_steps;) {
         const int left = n_steps - s;
         if (!recorded && (hybrid || by_three) && h->kind == 1 && left >= bc_graph_steps_of(by_three)) {
             if ((rc = bc_graph_steps(h, b, by_three))) return rc;
+            took(h, by_three ? 3 : 1, planes_wide);
             s += bc_graph_steps_of(by_three);
             continue;
         }
         if (by_three && h->kind == 1 && left >= 3) {
             CKL(launch_planes_x3(h, b, h->cur, h->stream), "d2q9_planes_x3");
+            took(h, 3, planes_wide);
             h->cur ^= 1;
             h->steps_done += 3;
             s += 3;
@@ -621,6 +678,7 @@ int advance(erlbm_handle *h, int n_steps, const BCp &b)
         if (plain && h->kind == 1 && (p.per_launch > 1 || p.fused1)) {
             if (!recorded && left >= graph_steps_of(p.per_launch)) {
                 if ((rc = graph_steps(h, p))) return rc;
+                took(h, p.per_launch, p.wide);
                 s += graph_steps_of(p.per_launch);
                 continue;
             }
@@ -630,6 +688,7 @@ int advance(erlbm_handle *h, int n_steps, const BCp &b)
             if (m > 1) {
                 CKL(launch_periodic(h, p, m, (const float *)h->d_buf[h->cur], (float *)h->d_buf[h->cur ^ 1], h->stream),
                     "periodic_d2q9");
+                took(h, m, m == 3 && p.wide);
                 h->cur ^= 1;
                 h->steps_done += m;
                 s += m;
@@ -893,7 +952,18 @@ int erlbm_step(erlbm_handle *h, int n_steps, const erlbm_bc *bc)
     if (n_steps < 0) return ERLBM_E_INVAL;
     BCp b;
     if ((rc = validate_bc(h, bc, &b))) return rc;
+    h->form_steps = 0;
     return advance(h, n_steps, b);
+}
+
+int erlbm_launch_form(const erlbm_handle *h, int *steps_per_launch, int *wide_strips)
+{
+    int rc = check_handle(h);
+    if (rc) return rc;
+    if (!steps_per_launch || !wide_strips) return ERLBM_E_INVAL;
+    *steps_per_launch = h->form_steps;
+    *wide_strips = h->form_steps > 0 && h->form_wide;
+    return ERLBM_OK;
 }
 
 int erlbm_set_launch(erlbm_handle *h, int block_threads, int flags)
@@ -998,6 +1068,7 @@ int erlbm_run(erlbm_handle *h, int n_steps, const erlbm_bc *bc, const erlbm_chec
     erlbm_checks c{};
     if (chk) c = *chk;
     if (c.energy_every < 0) return ERLBM_E_INVAL;
+    h->form_steps = 0;
     res->label = 0;
     res->decided_step = n_steps;
     res->steps_done = 0;

@@ -1252,13 +1252,13 @@ void go_planes_x3(const Geo &g, const BCp &bc, const shifted::Coef &k, const flo
 // From the sizes on where three steps by threes beat three single steps: a launch sequence costs three
 // latency-bound listed launches (about 5 us each), whatever the size, and saves two thirds of the traffic, or, where
 // nx % 128 != 0, the generic per-node kernel.  Measured on channels, us per step, single against threes:
-// fused single steps (nx % 128 == 0) 4096 x 1024 46.9 / 28.6, 2048 x 512 10.7 / 12.1, 1536 x 384 10.5 / 10.3, 512 x 128
-// 7.8 / 7.3; generic single steps 3000 x 1500 98.9 / 29.6, 2800 x 700 47.0 / 17.5, 1000 x 250 10.3 / 7.7, 500 x 125
-// 4.5 / 7.7.
+// fused single steps (nx % 128 == 0) 2048 x 512 10.5 / 12.4, 2304 x 576 13.1 / 16.2, 1536 x 1024 17.5 / 15.8, 2560 x 640 18.0 /
+// 15.8, 4096 x 1024 46.8 / 28.3; generic single steps 800 x 200 7.7 / 8.0, 1000 x 250 7.3 / 7.6, 1300 x 325 10.0 / 9.1,
+// 1500 x 375 12.0 / 9.7, 2000 x 500 18.2 / 12.3, 2800 x 700 42.7 / 17.2.
 bool d2q9_planes_x3_ok(const Geo &g)
 {
     return g.nz == 1 && g.nx >= 32 && g.ny >= 16 && g.nbox < (1LL << 31) - 256 &&
-           g.nbox >= (d2q9_hybrid_ok(g) ? 1500000 : 200000);
+           g.nbox >= (d2q9_hybrid_ok(g) ? 1500000 : 500000);
 }
 
 int d2q9_fix_distance(const Geo &g, const BCp &bc, uint8_t *fix, uint8_t *dist, cudaStream_t s)

@@ -133,6 +133,13 @@ int erlbm_get_populations(erlbm_handle *h, double *aos, size_t n, int stage);
 /* n_steps driver steps: [boundary planes] -> colisao_sitio at every node -> propag_site -> swap
  * (replaces e.g. main_double-shear-layer.cpp:382-449 without the output block).  bc may be NULL. */
 int erlbm_step(erlbm_handle *h, int n_steps, const erlbm_bc *bc);
+/* ERLBM_FP32_SHIFTED D2Q9 lattices take several steps per launch where that is faster, and replay blocks of
+ * steps as CUDA graphs; the results are those of single steps, bit for bit.  With solids or planes this needs
+ * a set-up: once calls in a row have asked for steps enough with the same planes (some 30 to 800, fewer for
+ * larger boxes), erlbm_step or erlbm_run waits for the handle's stream and allocates a third population buffer
+ * and a list of nodes, half as much device memory again, kept until erlbm_destroy; where memory is short the
+ * steps run one at a time as before.  Calls on a stream that is being captured do neither: they record plain
+ * launches. */
 /* kinectic_energy (Other_functions.cpp:100-115) of the chosen stage */
 int erlbm_kinetic_energy(erlbm_handle *h, int stage, double *energy);
 /* max over fluid nodes of |density| (LBM_functions.cpp:5544-5552) and a non-finite flag */
@@ -196,6 +203,9 @@ int erlbm_fp64_rate(double *ops_per_s);
 #define ERLBM_LAUNCH_THREE_STEP 4
 #define ERLBM_LAUNCH_WIDE_STRIPS 8
 int erlbm_set_launch(erlbm_handle *h, int block_threads, int flags);
+/* what the last erlbm_step or erlbm_run call did: the most steps that one of its launches took (1, 2 or 3; 0 before
+ * the first step), and whether in 64-column strips.  No counterpart in the reference. */
+int erlbm_launch_form(const erlbm_handle *h, int *steps_per_launch, int *wide_strips);
 /* run the handle's work on the caller's CUDA stream (a cudaStream_t; NULL = the handle's own
  * stream).  Waits for the work queued so far first.  No counterpart in the reference, whose loops
  * are synchronous; it lets a caller order the engine with its own GPU work and time it with events. */
