@@ -120,19 +120,18 @@ def peaks():
         return 6800.0, "fallback"
 
 
-def launches_of(n: int, per: int) -> int:
-    """Kernel launches of erlbm_step(n) on a lattice whose last step was a collision: blocks of 64 steps
-    (66 with three steps per launch) replayed as graphs, then multi-step launches, then single steps."""
-    g = 66 if per == 3 else 64
-    count, s = 0, 0
-    while s < n:
-        if n - s >= g:
-            count, s = count + g // per, s + g
-        elif per > 1 and n - s >= per:
-            count, s = count + 1, s + per
-        else:
-            count, s = count + 1, s + 1
-    return count
+def launches_of(n: int, per: int, own_shape: bool = False) -> int:
+    """Kernel launches of erlbm_step(n) on a periodic lattice whose last step was a collision: as many launches of
+    `per` steps as fit, then single steps, or one launch of two where the engine chose the shape (own_shape)."""
+    left = n % per
+    return n // per + (1 if own_shape and per == 3 and left == 2 else left)
+
+
+def fp64_kernel(op: int, mrt: int, n_nodes: int) -> str:
+    """The D2Q9 kernel that launch_step_fp64 takes."""
+    if op != mrt and n_nodes <= 7296:
+        return f"k_step_quad<9,{op}>"
+    return f"k_step<PrecExact64{'Small' if n_nodes < 32768 else ''},9,{op}>"
 
 
 def ncu_traffic(L: int, precision: str):
@@ -148,12 +147,13 @@ def ncu_traffic(L: int, precision: str):
         return None
 
 
-def channel_traffic(nx: int, ny: int):
-    """DRAM bytes per launch of the FP32 channel kernel from its committed ncu summary, scaled by the
-    box (the capture is of the bench's own 4096 x 1024 channel)."""
+def channel_traffic(nx: int, ny: int, per: int = 1):
+    """DRAM bytes per launch (per == 3: per sequence of launches that takes three steps) of the FP32 channel's
+    kernels from their committed ncu summary, scaled by the box (the capture is of the bench's own 4096 x 1024
+    channel)."""
     try:
         with open(os.path.join(ROOT, "profiles", "channel_step_traffic.json")) as f:
-            rec = json.load(f)["fp32"]
+            rec = json.load(f)["fp32_x3" if per == 3 else "fp32"]
         return (rec["dram_bytes_read"] + rec["dram_bytes_write"]) * (nx * ny) / (rec["nx"] * rec["ny"])
     except Exception:
         return None
@@ -375,9 +375,8 @@ def run_ours(args):
         t = torch.tensor([ms], device="cuda")
         dist.all_reduce(t, op=dist.ReduceOp.MAX)
         ms = float(t.item())
-    per = 3 if (shape and shape.get("three_step")) else (2 if (shape and shape.get("two_step")) else 1)
-    wide = bool(per == 3 and shape.get("wide_strips"))
-    launches = K * launches_of(inner, per)
+    per, wide = lat.launch_form()  # what the engine launched, whichever way the shape was chosen
+    launches = K * launches_of(inner, per, shape is None)
     value = world * L * L * inner * K / (ms / 1e3) / 1e6
     launch_ms = ms / launches
     algo_bytes = BYTES_PER_LU[args.precision] * L * L
@@ -445,7 +444,7 @@ def run_ours(args):
                      "kernel": (f"k_periodic_d2q9_x3a<{op}>" if wide else
                                 {1: f"k_periodic_d2q9<{op}>", 2: f"k_periodic_d2q9_x2s<{op}>",
                                  3: f"k_periodic_d2q9_x3s<{op}>"}[per])
-                     if args.precision == "fp32" else (f"k_step<PrecExact64,9,{op}>" if args.precision == "fp64"
+                     if args.precision == "fp32" else (fp64_kernel(op, E.OP_MRT, L * L) if args.precision == "fp64"
                                                        else f"k_step_pair<{op}>"),
                      # the update rate against the roofline of one step per launch, where every
                      # update reads and writes each population once (2 Q sizeof(real) bytes): the
@@ -474,13 +473,14 @@ def run_ours(args):
     return 0
 
 
-def fp64_ops_per_lu(L: int):
-    """FP64 add and multiply operations per lattice update of the plain kernel, from the committed ncu
-    instruction counts of the same kernel (profiles/dsl_periodic_d2q9_traffic.json, "fp64")."""
+def fp64_ops_per_lu(L: int, issued: bool = False):
+    """FP64 add and multiply operations that a lattice update of the plain path rounds, or, issued, those of them
+    that its kernel gives to the FP64 pipe, from the committed ncu instruction counts
+    (profiles/dsl_periodic_d2q9_traffic.json, "fp64")."""
     path = os.path.join(ROOT, "profiles", "dsl_periodic_d2q9_traffic.json")
     try:
         with open(path) as f:
-            return float(json.load(f)["fp64"]["fp64_ops_per_lu"])
+            return float(json.load(f)["fp64"]["fp64_pipe_ops_per_lu" if issued else "fp64_ops_per_lu"])
     except Exception:
         return None
 
@@ -527,18 +527,18 @@ def fp64_block(E, torch, L, f0, tau, op, tnh, K, W, inner):
     erlbm_fp64_rate) and against the HBM copy peak."""
     value, ms_step, launch_us, e2e = time_lattice(E, torch, L, f0, tau, op, tnh, K, W, inner, E.FP64)
     rate = E.fp64_rate()
-    ops = fp64_ops_per_lu(L)
+    ops = fp64_ops_per_lu(L, issued=True)
     hbm, hbm_kind = peaks()
     return {
         "lbm_steps_per_step": inner, "steps": K, "warmup": W,
         "value": value, "unit": "MLUPS", "dtype": "f64", "ms_per_step": ms_step,
-        "kernel": f"k_step<PrecExact64,9,{op}>",
+        "kernel": fp64_kernel(op, E.OP_MRT, L * L),
         "e2e": {"value": e2e, "unit": "MLUPS", "h2d_bytes_per_step": int(f0.nbytes), "d2h_bytes_per_step": 8},
         "roofline": {"bound": "fp64", "unit": "Gop/s",
                      "achieved": None if ops is None else ops * value * 1e6 / 1e9,
                      "peak": rate / 1e9, "peak_kind": "measured in this run (erlbm_fp64_rate: unfused DADD/DMUL)",
                      "frac": None if ops is None else ops * value * 1e6 / rate,
-                     "fp64_ops_per_lu": ops, "launch_us": launch_us},
+                     "fp64_ops_per_lu": ops, "rounded_ops_per_lu": fp64_ops_per_lu(L), "launch_us": launch_us},
         "hbm": {"bytes_per_lu": BYTES_PER_LU["fp64"], "achieved_gbs": value * 1e6 * BYTES_PER_LU["fp64"] / 1e9,
                 "peak_gbs": hbm, "frac": value * 1e6 * BYTES_PER_LU["fp64"] / 1e9 / hbm, "peak_kind": hbm_kind},
     }
@@ -975,7 +975,12 @@ def run_channel(args):
     clk = clocks.stop()
     ms = ev0.elapsed_time(ev1)
     value = n_fluid * inner * K / (ms / 1e3) / 1e6
-    launch_ms = ms / (K * inner)
+    # by threes, a sequence of four launches (the listed nodes' three steps, then the strips) takes three steps
+    per, wide = lat.launch_form()
+    launches = K * (4 * (inner // 3) + inner % 3 if per == 3 else inner)
+    launch_ms = ms / (K * inner) * per
+    kernel = ("k_step<PrecExact64,9,4>" if prec == E.FP64 else "k_d2q9_hybrid<4>" if per == 1 else
+              f"k_listed_step<4> x 3, k_periodic_d2q9_x3{'a' if wide else 's'}<4,SKIP>")
     bpl = BYTES_PER_LU["fp64" if prec == E.FP64 else "fp32"]
     peak, peak_kind = peaks()
     achieved = bpl * n_fluid / (launch_ms / 1e3) / 1e9
@@ -1020,13 +1025,14 @@ def run_channel(args):
                        "l2": f"working set {bpl * n_fluid / 1e6:.0f} MB (two population buffers) "
                              f"{'>' if bpl * n_fluid > 129e6 else '<'} 129 MB L2, no flush"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                         "peak_kind": peak_kind, "traffic": channel_traffic(nx, ny) if prec != E.FP64 else None,
+                         "peak_kind": peak_kind,
+                         "traffic": channel_traffic(nx, ny, per) if prec != E.FP64 else None,
                          "algorithmic_bytes_per_launch": bpl * n_fluid,
-                         "launch_us": launch_ms * 1e3, "lattice_updates_per_launch": n_fluid,
-                         "kernel": "k_step<PrecExact64,9,4>" if prec == E.FP64 else "k_d2q9_hybrid<4>"},
+                         "launch_us": launch_ms * 1e3, "lattice_updates_per_launch": n_fluid * per,
+                         "kernel": kernel},
             "e2e": {"value": n_fluid * inner * K / t_e2e / 1e6, "unit": "MLUPS",
                     "h2d_bytes_per_step": int(f0.nbytes), "d2h_bytes_per_step": 8},
-            "gpu_launches": K * inner, "clocks": clk}
+            "gpu_launches": launches, "clocks": clk}
     if cpu:
         line["cpu_baseline"] = cpu
     print(json.dumps(line))

@@ -2,7 +2,7 @@
 
 Two shapes are tuned by measurement on the GPU at hand:
   * the fused periodic D2Q9 FP32 kernel: threads per block (128 / 256 / 512), plain or streaming
-    (evict-first) stores, and one or two steps per launch, per lattice side L;
+    (evict-first) stores, and one, two or three steps per launch, per lattice side L;
   * the persistent map kernel: resident lattices ("slots") per SM, per map kind and precision.
 Each candidate is timed with CUDA events after a warm-up; the winner is cached in a JSON file
 ($ERLBM_TUNE_CACHE, default ~/.cache/erlbm_gb300/autotune.json) keyed by the device name, so later
@@ -59,17 +59,18 @@ def _time_steps(lat, stream, n: int) -> float:
 
 
 PERIODIC_CANDIDATES = [(128, False), (256, False), (512, False), (128, True), (256, True), (512, True)]
-# two and three steps per launch: one kernel shape each (warp strips in 128-thread CTAs); the block size
-# given with them is the one-step shape used for the steps a call has left over
+# two and three steps per launch: warp strips in 128-thread CTAs; the block size given with them is the one-step
+# shape used for the steps a call has left over.  Three steps without wide strips leave the strips' width to the
+# engine, so the last one is a candidate of its own only where that takes the 32-column ones.
 MULTI_STEP_CANDIDATES = [(128, False, 2), (128, False, 3), (128, True, 3)]  # (block, wide strips, steps)
 
 
 def tune_periodic(L: int, steps: int = 200, force: bool = False) -> dict:
-    """Best (block_threads, streaming_stores, two_step, three_step) of the fused D2Q9 FP32 kernel on an
-    L x L lattice."""
+    """Best (block_threads, streaming_stores, two_step, three_step, wide_strips) of the fused D2Q9 FP32 kernel on
+    an L x L lattice."""
     import torch
     import erlbm_gb300 as E
-    key = f"{_device_key()}/periodic_d2q9_fp32/shapes4/L{L}"
+    key = f"{_device_key()}/periodic_d2q9_fp32/shapes5/L{L}"
     hit = _load().get(key)
     if hit and not force:
         return hit
@@ -84,10 +85,14 @@ def tune_periodic(L: int, steps: int = 200, force: bool = False) -> dict:
         cands = [(b, s, False, 1) for b, s in PERIODIC_CANDIDATES]
         if L % 2 == 0 and L >= 4:
             cands += [(b, False, w, per) for b, w, per in MULTI_STEP_CANDIDATES if not w or L >= 16]
+        engine_wide = False
         for block, st, wide, per in cands:
+            if wide and engine_wide:
+                continue
             lat.set_launch(block, st, per == 2, per == 3, wide)
             lat.step(20)
             t = min(_time_steps(lat, stream, steps) for _ in range(3))
+            engine_wide = lat.launch_form() == (3, True)
             results.append(dict(block_threads=block, streaming_stores=st, two_step=per == 2, three_step=per == 3,
                                 wide_strips=wide, mlups=L * L * steps / t / 1e6))
     best = max(results, key=lambda r: r["mlups"])
