@@ -1,7 +1,7 @@
 // fp64_int.cuh -- parts of the exact FP64 collision on the integer pipes, with the FP64 pipe's bits.
 //
-// GB300 issues two FP64 operations per clock and SM (a warp instruction holds its scheduler's FP64 pipe for 64
-// cycles), but 64 integer ALU operations and 64 integer multiply-adds.  Where the range of the operands is known,
+// GB300 issues fewer than two FP64 operations per clock and SM (a warp instruction holds its scheduler's FP64 pipe for
+// some 80 cycles), but 64 integer ALU operations and 64 integer multiply-adds.  Where the range of the operands is known,
 // a correctly rounded FP64 add is an integer add and a rounding to a fixed bit position, about a dozen integer
 // instructions, and runs beside the FP64 work of the other warps.  Everything here is integer arithmetic from the
 // definition of round-to-nearest-even; the results are the IEEE ones, bit for bit.

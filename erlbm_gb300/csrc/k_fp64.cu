@@ -5,10 +5,9 @@
 
 namespace erlbm {
 
-// From this size on (past QUAD_MAX_NODES: the small sizes below are those of one lane a node) every scheduler has two
-// warps or more, and the fixed-point sums of the collision cost
-// less than the FP64 operations they replace; below, a warp waits for its own integer chains.  us per step without
-// and with: D3Q19 16^3 14.4 / 18.5, 24^3 15.4 / 18.5, 32^3 23.7 / 22.6, 64^3 135.7 / 114.9; D2Q9 160^2 10.3 / 10.3,
+// From this size on every scheduler has two warps or more, and the fixed-point sums of the collision cost less than
+// the FP64 operations they replace; below, a warp waits for its own integer chains.  us per step without and with, one
+// lane a node: D3Q19 16^3 14.4 / 18.5, 24^3 15.4 / 18.5, 32^3 23.7 / 22.6, 64^3 135.7 / 114.9; D2Q9 160^2 10.3 / 10.3,
 // 200^2 16.3 / 13.4, 512^2 65.7 / 49.2.
 constexpr long long FIXED_MIN_NODES = 32768;
 

@@ -5,9 +5,10 @@ namespace erlbm {
 
 namespace {
 
-// Both map lattices have 256 fluid nodes.  Bounded to 256 threads, two CTAs an SM leave 128 registers a thread; with
-// 288, nine warps a CTA, they leave 96 and the exact D3Q19 collision spills 964 bytes instead of 444.  600
-// obstacle runs of 1000 steps: 117.2 -> 112 ms with the fixed-point sums of the collision, 113.8 without them.
+// The Taylor-Green map's lattice has 256 fluid nodes, the obstacle map's 232.  Bounded to 256 threads, two CTAs an SM
+// leave 128 registers a thread; with 288, nine warps a CTA, they leave 96 and the exact D3Q19 collision stores 728 bytes
+// of spills instead of 468.  600 obstacle runs of 1000 steps when the bound came in: 117.2 -> 112 ms with the fixed-point
+// sums of the collision, 113.8 without them (76.7 now; without 113).
 constexpr int MAP_THREADS = 256;
 
 template <int Q, int NPT, int MAXT = BatchBounds<NPT, 8>::MAXT>
