@@ -429,8 +429,8 @@ def run_ours(args):
         "config": {"workload": f"double shear layer D2Q9 {op_label} Re=80000 L={L}, "
                                f"{dict(fp32='FP32-shifted', fp64='FP64 plain', pair='compensated FP32 pairs')[args.precision]}",
                    "L": L, "lbm_steps_per_step": inner, "parallelism": f"replicas x{world}",
-                   "l2": f"working set {2 * BYTES_PER_LU[args.precision] // 2 * L * L / 1e6:.0f} MB > 129 MB L2, "
-                         "no flush",
+                   "l2": f"working set {2 * BYTES_PER_LU[args.precision] // 2 * L * L / 1e6:.0f} MB "
+                         f"{'>' if BYTES_PER_LU[args.precision] * L * L > 129e6 else '<'} 129 MB L2, no flush",
                    "launch_shape": None if shape is None else {"block_threads": shape["block_threads"],
                                                                "streaming_stores": shape["streaming_stores"],
                                                                "steps_per_launch": per, "wide_strips": wide}},

@@ -116,7 +116,7 @@ def tune_map(kind: int, precision: int, map_points: int = 40, max_steps: int = 3
     import time
     import torch
     import erlbm_gb300 as E
-    key = f"{_device_key()}/map/{kind}/{precision}"
+    key = f"{_device_key()}/map2/{kind}/{precision}"
     hit = _load().get(key)
     if hit and not force:
         return hit
@@ -143,7 +143,7 @@ def tune_map(kind: int, precision: int, map_points: int = 40, max_steps: int = 3
 def best_slots(kind: int, precision: int) -> int:
     """Cached slots per SM for a map kind and precision, 0 (as many as fit) if none is cached."""
     try:
-        hit = _load().get(f"{_device_key()}/map/{kind}/{precision}")
+        hit = _load().get(f"{_device_key()}/map2/{kind}/{precision}")
     except Exception:
         hit = None
     return int(hit["slots"]) if hit else 0
