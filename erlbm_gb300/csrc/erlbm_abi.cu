@@ -159,14 +159,29 @@ void drop_graphs(erlbm_handle *h)
     drop_bc_graphs(h);
 }
 
+// Buffers that a step call takes and gives back: in stream order, because cudaFree waits for the whole device, and with
+// it for the server's resident loops.
+template <class T>
+bool take(erlbm_handle *h, T *&p, size_t bytes)
+{
+    if (p) return true;
+    if (cudaMallocAsync((void **)&p, bytes, h->stream) == cudaSuccess) return true;
+    cudaGetLastError();
+    p = nullptr;
+    return false;
+}
+template <class T>
+void give_back(erlbm_handle *h, T *&p)
+{
+    if (p) cudaFreeAsync(p, h->stream);
+    p = nullptr;
+}
+
 void drop_planes_x3(erlbm_handle *h)
 {
-    cudaFree(h->d_x3_dist);
-    cudaFree(h->d_x3_list);
-    cudaFree(h->d_x3_mid);
-    h->d_x3_dist = nullptr;
-    h->d_x3_list = nullptr;
-    h->d_x3_mid = nullptr;
+    give_back(h, h->d_x3_dist);
+    give_back(h, h->d_x3_list);
+    give_back(h, h->d_x3_mid);
     h->x3_state = 0;
 }
 
@@ -177,7 +192,9 @@ void free_handle(erlbm_handle *h)
     cudaFree(h->d_segflag);
     cudaFree(h->d_nodeflag);
     cudaFree(h->d_fix);
-    drop_planes_x3(h);
+    cudaFree(h->d_x3_dist);
+    cudaFree(h->d_x3_list);
+    cudaFree(h->d_x3_mid);
     cudaFree(h->d_profile);
     cudaFree(h->d_nof);
     cudaFree(h->d_buf[0]);
@@ -512,14 +529,8 @@ int setup_planes_x3(erlbm_handle *h, const BCp &b)
     memcpy(h->x3_planes, planes, sizeof(planes));
     h->x3_state = 0;
     h->x3_asked = 0;
-    cudaFree(h->d_x3_list);
-    h->d_x3_list = nullptr;
-    auto no_memory = [h] {
-        cudaGetLastError();
-        drop_planes_x3(h);
-        return ERLBM_OK;
-    };
-    if (!h->d_x3_dist && cudaMalloc(&h->d_x3_dist, 2 * h->g.nbox) != cudaSuccess) return no_memory();
+    give_back(h, h->d_x3_list);
+    if (!take(h, h->d_x3_dist, 2 * h->g.nbox)) return drop_planes_x3(h), ERLBM_OK;
     uint8_t *fix = h->d_x3_dist + h->g.nbox;
     int *at = (int *)h->d_out, *n = h->x3_listed;
     CK(cudaMemsetAsync(at, 0, 3 * sizeof(int), h->stream));
@@ -533,14 +544,9 @@ int setup_planes_x3(erlbm_handle *h, const BCp &b)
         h->x3_state = -1;
         return ERLBM_OK;
     }
-    if (cudaMalloc(&h->d_x3_list, (all > 0 ? all : 1) * sizeof(int)) != cudaSuccess) {
-        h->d_x3_list = nullptr;
-        return no_memory();
-    }
-    if (!h->d_x3_mid && cudaMalloc(&h->d_x3_mid, (size_t)h->q * h->g.plane * sizeof(float)) != cudaSuccess) {
-        h->d_x3_mid = nullptr;
-        return no_memory();
-    }
+    if (!take(h, h->d_x3_list, (all > 0 ? all : 1) * sizeof(int)) ||
+        !take(h, h->d_x3_mid, (size_t)h->q * h->g.plane * sizeof(float)))
+        return drop_planes_x3(h), ERLBM_OK;
     const int from[3] = {0, n[0], n[0] + n[1]};
     CK(cudaMemcpyAsync(at, from, sizeof(from), cudaMemcpyHostToDevice, h->stream));
     CKL(d2q9_fix_list(h->g, fix, h->d_x3_dist, at, h->d_x3_list, h->stream), "fix_list");

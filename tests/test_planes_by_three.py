@@ -120,3 +120,30 @@ def test_launch_shapes_asked_for_on_boxes_of_any_size(nx, ny, steps):
             lat.set_populations(f)
             lat.step(steps)
             assert np.array_equal(lat.get_populations(E.STAGE_POST_COLLISION), want), shape
+
+
+def test_set_ups_do_not_wait_for_the_servers_resident_loops():
+    """While a server works through a long request: a set-up, one that replaces it and one that is refused."""
+    import erlbm_gb300 as E
+    nx, ny = 1660, 922
+    a, b = pair(E, nx, ny, geometry(nx, ny, 8))
+    c, d = pair(E, 1003, 700, geometry(1003, 700, 9, scattered=20000))
+    with a, b, c, d, E.Server(hbm_budget_bytes=1 << 30) as srv:
+        def run(steps):
+            return srv.submit(E.REQ_TG3D, E.FP64, E.OP_EXTREG, L=64, tau=0.55, tau_nh=0.65, u0=0.05, n_steps=steps)
+        srv.wait(run(2))
+        ticket = run(30000)  # some seconds
+        for kind in ("channel", "open"):
+            a.step(100, planes(E, nx, ny, kind))
+            a.sync()
+            assert a.launch_form()[0] == 3
+        c.step(400, planes(E, 1003, 700, "channel"))
+        c.sync()
+        assert c.launch_form() == (1, False)
+        assert srv.poll(ticket) is None  # still running
+        for kind in ("channel", "open"):
+            for _ in range(100):
+                b.step(1, planes(E, nx, ny, kind))
+        b.sync()
+        assert srv.wait(ticket)["status"] == 0
+        assert same(E, a, b)
