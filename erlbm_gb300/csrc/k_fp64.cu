@@ -147,6 +147,10 @@ constexpr int SER_THREADS = 32 * SER_WARPS;
 constexpr int SER_PER_LANE = 8;
 constexpr int SER_CHUNK = SER_THREADS * SER_PER_LANE;
 constexpr int SER_STOPS = 34;
+// Up to this length the plain loop is as fast: the first terms leave the sum's binade one after the other, a pass over
+// the chunk each.  us of erlbm_kinetic_energy by the loop and by passes: FP64 16 nodes 22 / 30, 144 30 / 45, 256 32 / 48,
+// 484 43 / 56, 576 56 / 56; FP32 484 43 / 43, 784 58 / 44.
+constexpr int SER_PLAIN = 512;
 
 __global__ void __launch_bounds__(SER_THREADS) k_sum_serial(const double *__restrict__ x, long long n, double *out)
 {
@@ -157,6 +161,12 @@ __global__ void __launch_bounds__(SER_THREADS) k_sum_serial(const double *__rest
     __shared__ int stop_at[2][SER_WARPS];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double s = 0.0;  // the same in every thread
+    if (n <= SER_PLAIN) {
+        if (tid != 0) return;
+        for (long long i = 0; i < n; i++) s = s + x[i];
+        *out = s;
+        return;
+    }
     double v[SER_PER_LANE], nx[SER_PER_LANE];
     auto load = [&](long long base, double w[SER_PER_LANE]) {
 #pragma unroll
